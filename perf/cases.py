@@ -393,6 +393,16 @@ def _run_adjoint(s):
     return [s.x, s.gb, s.gA]
 
 
+class _Held(np.ndarray):
+    """An array in memory that the library allocated, which its owner releases."""
+
+
+def _values(M):
+    v = np.ctypeslib.as_array(C.cast(M.m.val, C.POINTER(C.c_double)), shape=(M.m.nnz,)).view(_Held)
+    v.owner = M
+    return v
+
+
 def _run_dropin(s):
     from lace_gb300 import dropin
     c = s.case
@@ -401,8 +411,7 @@ def _run_dropin(s):
     s.x[:] = 0.0
     x, rc, log = dropin.fgmres_householder_restart(s.A, s.b, s.x, L, U, search_max=c["m"], restart_max=60,
                                                    rtol=c["rtol"], tol_type=1, x0_inplace=True)
-    s.L, s.U = L, U  # the program's factors, released when it has new ones
-    vals = [np.ctypeslib.as_array(C.cast(M.m.val, C.POINTER(C.c_double)), shape=(M.m.nnz,)) for M in (L, U)]
+    vals = [_values(M) for M in (L, U)]
     return [x, *vals]
 
 
