@@ -423,8 +423,10 @@ int lace_gpu_apply_precond(lace_gpu_ctx *ctx, const double *q, double *z);
 
 /* The sync-free solve schedule in use, once the first solve has tuned it:
  * out[0] rows per lane, out[1] chunks per block, out[2] warps per CTA,
- * out[3] CTAs per thread-block cluster (1: none).  DEV_ERR_NOT_INITIALIZED
- * before.  No counterpart in LACE. */
+ * out[3] CTAs per thread-block cluster (1: none).  For the factors of a 5- or
+ * 7-point grid in natural order, solved a lane per grid line: out[0] the rows
+ * of a line, out[1] and out[2] the tiles (warps) per CTA, out[3] as above.
+ * DEV_ERR_NOT_INITIALIZED before.  No counterpart in LACE. */
 int lace_gpu_get_trsv_schedule(lace_gpu_ctx *ctx, int *out);
 
 /* z = M^{-1} q as one step of the FGMRES cycle applies it, enqueued on the

@@ -9,7 +9,9 @@
 //          plus its CSR form (diagonal first) for the solves, with a position
 //          map csr->csc (the CSR values are gathered after the sweeps)
 //   L^T    CSR of L's transpose (adjoint solves), with a position map
-//   per triangle: chunk kinds (u8), ready flags (i32), level lists (i32)
+//   per triangle: chunk kinds (u8), ready flags (i32), level lists (i32); on a
+//          grid stencil instead the values in the order its lanes use them
+//          (sptrsv_grid.cu)
 //   Krylov V[ldv x (m+1)] f64 column-major (ldv = n rounded up to 32, plus
 //          32 so that columns are not a power of two bytes apart),
 //          Z[ldv x m] f32 (mixed precision) or f64, w/q/t vectors
@@ -459,6 +461,7 @@ using namespace lace;
 // the block-scheduled plan of one triangle with the current schedule shape,
 // its values gathered from the current factor values
 int lace_gpu_ctx::ensure_plan(int which) {
+  if (grid_on) return ensure_grid(which);
   PlanBufs &pb = plans[which];
   TriDev t = tri(which);
   if (!(pb.valid && pb.dev.R == plan_R && pb.dev.cpb == plan_cpb)) {
@@ -486,6 +489,71 @@ int lace_gpu_ctx::ensure_plan(int which) {
     pb.vals_type = (int)vtype();
     pb.vals_src = t.val;
   }
+  return cudaGetLastError() == cudaSuccess ? 0 : DEV_ERR_UNKNOWN;
+}
+
+// Whether the factors are those of a grid stencil, by L's last row and then,
+// on the device, by every row of L and U; their transposes then are, too.  A
+// pinned schedule keeps the block-scheduled solves.
+int lace_gpu_ctx::try_grid() {
+  grid_on = false;
+  for (auto &p : gplans) p.valid = false;
+  if (bs || opt.trsv_chunks_per_block > 0 || opt.trsv_rows_per_lane > 0 || n < 2) return 0;
+  int d[3] = {0, 0, 0};
+  const int off = hL.ptr[n] - 1 - hL.ptr[n - 1];  // L's last row without its diagonal
+  if (off < 2 || off > 3) return 0;
+  for (int k = 0; k < off; ++k) d[k] = n - 1 - hL.idx[hL.ptr[n] - 2 - k];
+  const size_t ct = vtype() == VType::F64 ? 8 : 4;
+  if (!grid_shape(n, d[0], d[1], d[2], ct, grid)) return 0;
+  int *flag = (int *)cnt_buf.p + 48;
+  for (int w = 0; w < 2; ++w) {
+    const TriDev t = tri(w);
+    bool ok = false;
+    const int rc = grid_check(stream, grid, w == 0, t.row, t.col, flag, &ok);
+    if (rc) return rc;
+    if (!ok) return 0;
+  }
+  if (grid_t.ensure(ct * grid.vec())) return DEV_ERR_DEVICE_ALLOC;
+  if (cudaMemsetAsync(grid_t.p, 0, ct * grid.vec(), stream) != cudaSuccess) return DEV_ERR_UNKNOWN;
+  grid_on = true;
+  return 0;
+}
+
+int lace_gpu_ctx::ensure_grid(int which) {
+  GridPlan &p = gplans[which];
+  const TriDev t = tri(which);
+  if (!p.valid) {
+    const int rc = grid_prepare(stream, grid, t.lower != 0, t.unit != 0, vtype(), p);
+    if (rc) return rc;
+  }
+  if (p.vals_version != fact_version || p.vals_src != t.val) {
+    launch_grid_values(stream, p, t.row, t.col, t.val, vtype());
+    p.vals_version = fact_version;
+    p.vals_src = t.val;
+  }
+  return cudaGetLastError() == cudaSuccess ? 0 : DEV_ERR_UNKNOWN;
+}
+
+int lace_gpu_ctx::limit_reached() {
+  for (auto &p : gplans)
+    if (p.valid) grid_clear_faces(stream, p);
+  return DEV_ERR_INTERNAL_LIMIT;
+}
+
+int lace_gpu_ctx::solve_pair(int t1, int t2, const void *b, int in_f32, void *z, int z_f32, bool honor_done,
+                             bool prefilled) {
+  const int f32 = vtype() != VType::F64;  // the vector between the triangles
+  if (!(grid_on && syncfree_blocks())) {
+    const int rc = solve_tri(t1, b, in_f32, vec_t.p, f32, honor_done, vec_t2.p, prefilled);
+    return rc ? rc : solve_tri(t2, vec_t.p, f32, z, z_f32, honor_done, vec_t2.p, prefilled);
+  }
+  int rc = ensure_grid(t1);
+  if (!rc) rc = ensure_grid(t2);
+  Control *cb = ctrl();
+  if (!rc)
+    rc = launch_grid_pair(stream, gplans[t1], gplans[t2], b, in_f32, grid_t.p, z, z_f32, &cb->status,
+                          honor_done ? &cb->done : nullptr);
+  if (rc) return rc;
   return cudaGetLastError() == cudaSuccess ? 0 : DEV_ERR_UNKNOWN;
 }
 
@@ -1509,6 +1577,12 @@ int lace_gpu_ctx::solve_tri(int which, const void *b, int in_f32, void *x, int o
       } else {
         int rc = ensure_plan(which);
         if (rc) return rc;
+        if (grid_on) {
+          rc = launch_grid_tri(stream, gplans[which], b, in_f32, grid_t.p, x, out_f32, &cb->status,
+                               honor_done ? &cb->done : nullptr);
+          if (rc) return rc;
+          break;
+        }
         if (b == x) {  // the solve fills x before it reads b
           cudaMemcpyAsync(tmp, b, (size_t)n * (in_f32 ? 4 : 8), cudaMemcpyDeviceToDevice, stream);
           b = tmp;
@@ -1578,7 +1652,13 @@ int lace_gpu_ctx::autotune_trsv() {
   if (bs || opt.trsv_mode != LACE_TRSV_SYNCFREE) return 0;
   if (trsv_tuned) return 0;
   int rc = ensure_vectors();
+  if (!rc) rc = try_grid();
   if (rc) return rc;
+  if (grid_on) {
+    trsv_tuned = true;
+    drop_graphs();
+    return 0;
+  }
   const bool f32 = vtype() != VType::F64;
   cudaMemsetAsync(vec_q.p, 0, 8 * (size_t)n, stream);
   cudaEvent_t e0, e1;
@@ -1777,7 +1857,7 @@ extern "C" int lace_gpu_sptrsv(lace_gpu_ctx *c, int which, const double *b, doub
   if (rc) return set_err(rc);
   LCHK(cudaStreamSynchronize(c->stream));
   int st = c->h_status();
-  if (st & kStatusSpinTimeout) return set_err(DEV_ERR_INTERNAL_LIMIT);
+  if (st & kStatusSpinTimeout) return set_err(c->limit_reached());
   return DEV_SUCCESS;
 }
 
@@ -1786,14 +1866,19 @@ extern "C" int lace_gpu_precond_enqueue(lace_gpu_ctx *c, const void *q, void *z)
   if (!c->factors_ready || !c->trsv_tuned) return set_err(DEV_ERR_NOT_INITIALIZED);
   cudaSetDevice(c->device);
   const int f32 = c->vtype() != VType::F64;
-  int rc = c->solve_tri(0, q, f32, c->vec_t.p, f32, false, c->vec_t2.p);
-  if (!rc) rc = c->solve_tri(1, c->vec_t.p, f32, z, f32, false, c->vec_t2.p);
+  const int rc = c->solve_pair(0, 1, q, f32, z, f32, false, false);
   return rc ? set_err(rc) : DEV_SUCCESS;
 }
 
 extern "C" int lace_gpu_get_trsv_schedule(lace_gpu_ctx *c, int *out) {
   if (!c || !out) return set_err(DEV_ERR_INVALID_PTR);
   if (!c->trsv_tuned) return set_err(DEV_ERR_NOT_INITIALIZED);
+  if (c->grid_on) {  // a lane per line of the grid, a warp per tile of lines
+    out[0] = c->grid.nx;
+    out[1] = out[2] = c->grid.wy * c->grid.wz;
+    out[3] = c->grid.cy * c->grid.cz;
+    return DEV_SUCCESS;
+  }
   out[0] = c->plan_R;
   out[1] = c->plan_cpb;
   out[2] = c->plan_warps;
@@ -1810,18 +1895,15 @@ extern "C" int lace_gpu_apply_precond(lace_gpu_ctx *c, const double *q, double *
   if (rc) return set_err(rc);
   cudaMemsetAsync(&c->ctrl()->status, 0, 4, c->stream);
   const int f32 = c->vtype() != VType::F64;
-  rc = c->solve_tri(0, q, 0, c->vec_t.p, f32, false, c->vec_t2.p);
-  if (!rc) {
-    if (f32) {
-      rc = c->solve_tri(1, c->vec_t.p, 1, c->vec_r.p, 1, false, c->vec_t2.p);
-      launch_convert(c->stream, c->n, VType::F32, c->vec_r.p, VType::F64, z);
-    } else {
-      rc = c->solve_tri(1, c->vec_t.p, 0, z, 0, false, c->vec_t2.p);
-    }
+  if (f32) {
+    rc = c->solve_pair(0, 1, q, 0, c->vec_r.p, 1, false, false);
+    if (!rc) launch_convert(c->stream, c->n, VType::F32, c->vec_r.p, VType::F64, z);
+  } else {
+    rc = c->solve_pair(0, 1, q, 0, z, 0, false, false);
   }
   if (rc) return set_err(rc);
   LCHK(cudaStreamSynchronize(c->stream));
-  if (c->h_status() & kStatusSpinTimeout) return set_err(DEV_ERR_INTERNAL_LIMIT);
+  if (c->h_status() & kStatusSpinTimeout) return set_err(c->limit_reached());
   return DEV_SUCCESS;
 }
 
@@ -1964,7 +2046,7 @@ ArnoldiArgs lace_gpu_ctx::arnoldi_args(int m, bool adjoint) {
   a.cy = (Cycle *)cycle_buf.p;
   a.ctrl = ctrl();
   a.m = m;
-  a.prefill = syncfree_blocks() ? 1 : 0;
+  a.prefill = syncfree_blocks() && !grid_on ? 1 : 0;
   a.fill_t = vec_t.p;
   a.fill_t_f32 = vtype() != VType::F64 ? 1 : 0;
   return a;
@@ -1973,12 +2055,10 @@ ArnoldiArgs lace_gpu_ctx::arnoldi_args(int m, bool adjoint) {
 // the search-direction loop of one cycle (LACE :311-759), all on the device
 int lace_gpu_ctx::enqueue_cycle_body(const ArnoldiArgs &a, int m, bool adjoint, bool capturing) {
   const int t1 = adjoint ? 2 : 0, t2 = adjoint ? 3 : 1;
-  const int tf32 = vtype() != VType::F64;  // the intermediate vector of the two solves
   for (int j = 0; j < m; ++j) {
     void *zj = (char *)a.Z + (size_t)j * a.ldz * (a.z_f32 ? 4 : 8);
     // both outputs were marked unsolved by the kernel before (a.prefill)
-    int rc = solve_tri(t1, a.q, a.q_f32, vec_t.p, tf32, true, vec_t2.p, a.prefill != 0);
-    if (!rc) rc = solve_tri(t2, vec_t.p, tf32, zj, a.z_f32, true, vec_t2.p, a.prefill != 0);
+    int rc = solve_pair(t1, t2, a.q, a.q_f32, zj, a.z_f32, true, a.prefill != 0);
     if (rc) return rc;
     // passes A, B and C as one cooperative kernel where it applies
     const int st = hh_persistent ? launch_hh_step(stream, a, j) : 1;
@@ -2005,15 +2085,13 @@ int lace_gpu_ctx::enqueue_cycle_body(const ArnoldiArgs &a, int m, bool adjoint, 
 // the modified Gram-Schmidt search-direction loop of one cycle
 // (src/fgmres_restart.cpp:227-494), all on the device
 int lace_gpu_ctx::enqueue_mgs_body(const ArnoldiArgs &a, int m, bool capturing) {
-  const int tf32 = vtype() != VType::F64;
   // LACE's test reorthogonalises for reorth 0 (when needed) and 2 (always)
   const bool second = a.mgs_reorth == 0 || a.mgs_reorth == 2;
   for (int j = 0; j < m; ++j) {
     void *zj = (char *)a.Z + (size_t)j * a.ldz * (a.z_f32 ? 4 : 8);
     const double *vj = a.V + (size_t)j * a.ldv;
     // z_j = U^{-1} L^{-1} v_j (:239-270); outputs marked unsolved before
-    int rc = solve_tri(0, vj, 0, vec_t.p, tf32, true, vec_t2.p, a.prefill != 0);
-    if (!rc) rc = solve_tri(1, vec_t.p, tf32, zj, a.z_f32, true, vec_t2.p, a.prefill != 0);
+    int rc = solve_pair(0, 1, vj, 0, zj, a.z_f32, true, a.prefill != 0);
     if (rc) return rc;
     // the whole step as one cooperative kernel where it applies
     const int st = mgs_persistent ? launch_mgs_step(stream, a, j) : 1;
@@ -2206,7 +2284,7 @@ int lace_gpu_ctx::fgmres(const double *b, double *x, int m, int restart_max, int
       memcpy(&nr, h_scal + kScalReorth, 4);
       last_reorth += nr;
     }
-    if (hc.status & kStatusSpinTimeout) return DEV_ERR_INTERNAL_LIMIT;
+    if (hc.status & kStatusSpinTimeout) return limit_reached();
     const int ns = hc.nsteps;
     if (capped && ns == m && !hc.converged && !(hc.status & kStatusBreakdown)) return DEV_ERR_NOT_SUPPORTED;
     if (hist)

@@ -38,6 +38,31 @@ struct PlanBufs {
   const void *vals_src = nullptr;
 };
 
+// one triangle's plan on a grid stencil (sptrsv_grid.cu).  coef: per tile,
+// block of four steps and coefficient, four values per lane; face: per tile LZ
+// rows towards the previous tile in y and LY rows towards the previous tile in
+// z, 4 nb entries each, unsolved between solves; ctl: tickets, and whether a
+// wait gave up
+struct GridPlan {
+  bool valid = false;
+  GridShape g;
+  int lower = 1, unit = 0;
+  size_t ct = 4;
+  DBuf coef, face, ctl;
+  int vals_version = -1;
+  const void *vals_src = nullptr;
+};
+int grid_prepare(cudaStream_t s, const GridShape &g, bool lower, bool unit, VType vt, GridPlan &p);
+int grid_clear_faces(cudaStream_t s, GridPlan &p);
+void launch_grid_values(cudaStream_t s, GridPlan &p, const int *row, const int *col, const void *val, VType vt);
+// x = T2^{-1} T1^{-1} b, T1 lower and T2 upper on the same grid, and x = T^{-1} b;
+// t: a vector in tile order (GridShape::vec elements of the compute type, zero
+// in its padding)
+int launch_grid_pair(cudaStream_t s, GridPlan &p1, GridPlan &p2, const void *b, int in_f32, void *t, void *x, int out_f32,
+                     int *status, const int *done);
+int launch_grid_tri(cudaStream_t s, GridPlan &p, const void *b, int in_f32, void *t, void *x, int out_f32, int *status,
+                    const int *done);
+
 // host part of a plan (what build_blk_plan_host fills, upload_blk_plan sends)
 struct HostPlan {
   int n = 0, nch = 0, R = 1, cpb = 1, max_units = 0;
@@ -121,6 +146,16 @@ struct lace_gpu_ctx {
   lace::PlanBufs plans[4];
   int plan_R = 4, plan_cpb = 1, plan_warps = 1, plan_cl = 1;  // autotuned schedule shape
   int ensure_plan(int which);
+  // the solves of a grid stencil (sptrsv_grid.cu), chosen by try_grid
+  bool grid_on = false;
+  lace::GridShape grid;
+  lace::GridPlan gplans[4];
+  lace::DBuf grid_t;  // the vector between the two triangles, in tile order
+  int try_grid();
+  int ensure_grid(int which);
+  int limit_reached();  // DEV_ERR_INTERNAL_LIMIT, after making the grid plans usable again
+  // z = T2^{-1} T1^{-1} b for two consecutive triangles (L and U, or U^T and L^T)
+  int solve_pair(int t1, int t2, const void *b, int in_f32, void *z, int z_f32, bool honor_done, bool prefilled);
   // host plans the autotune built in parallel, keyed (triangle, R, chunks per block)
   std::map<std::tuple<int, int, int>, lace::HostPlan> prebuilt;
   int lanes = 8;

@@ -324,6 +324,42 @@ void launch_sptrsv_blk_multi(cudaStream_t s, const TriBlkPlan &pl, const void *v
                              int in_f32, void *x, int out_f32, size_t vstride, int nrhs, int *tickets, int *status,
                              const int *done_flag, bool prefilled = false);
 
+// Grid stencils (sptrsv_grid.cu): the box of lines a triangle's rows form, cut
+// into tiles of 2^lyl x (32 >> lyl) lines (a warp each), super-tiles of wy x wz
+// tiles (a CTA each; sy x sz of them, in clusters of cy x cz) and nb blocks of
+// four steps along x
+struct GridShape {
+  int nx = 0, ny = 0, nz = 0;
+  int lyl = 0, wy = 1, wz = 1, cy = 1, cz = 1, sy = 0, sz = 0, nb = 0;
+  // coefficients per row: x, y, [z], [the reciprocal diagonal]
+  __host__ __device__ int coefs(int unit) const { return (nz > 1 ? 4 : 3) - (unit ? 1 : 0); }
+  __host__ __device__ int tiles() const { return sy * wy * sz * wz; }
+  // rows of a tile's faces: its first lines in y, its first in z
+  __host__ __device__ int face_rows() const { return (32 >> lyl) + (nz > 1 ? 1 << lyl : 0); }
+  // elements of a vector in tile order
+  __host__ __device__ size_t vec() const { return (size_t)tiles() * nb * 128; }
+  // the step at which the first line of tile (ty, tz) starts: 0 to 3 for a lower
+  // triangle, so that a tile's block of four steps takes whole blocks of its
+  // neighbours' results (their first lines are LY - 1 or LZ - 1 steps before
+  // their last); an upper triangle's tiles (counted from the other end) walk
+  // the lower's backwards, step t there being step 4 nb - 1 - t here
+  __host__ __device__ int first(bool lower, int ty, int tz) const {
+    const int LY = 1 << lyl, LZ = 32 >> lyl;
+    if (!lower) {
+      ty = sy * wy - 1 - ty;
+      tz = sz * wz - 1 - tz;
+    }
+    const int f = ((LY - 1) * ty + (LZ - 1) * tz) & 3;
+    return lower ? f : 4 * nb - (nx + LY + LZ - 2) - f;
+  }
+};
+// the shape of an n-row box whose last row's neighbours are d1 < d2 [< d3]
+// rows away (d3 0: none); false when those are not whole lines and planes, do
+// not fit, or are faster by blocks of chunks (ct: bytes of the compute type)
+bool grid_shape(int n, int d1, int d2, int d3, size_t ct, GridShape &g);
+// *ok: every row of the triangle has exactly the neighbours of its place in the box
+int grid_check(cudaStream_t s, const GridShape &g, bool lower, const int *row, const int *col, int *flag, bool *ok);
+
 // honor_done: return at once when ctrl->done is set (inside an Arnoldi cycle)
 void launch_sptrsv_levels(cudaStream_t s, const TriDev &t, VType vt, const void *b, int in_f32,
                           void *x, int out_f32, Control *ctrl, bool honor_done);
