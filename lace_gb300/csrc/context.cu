@@ -1934,6 +1934,11 @@ int lace_gpu_ctx::ensure_krylov(int m, bool monitor) {
     if (Qmon.ensure(8 * ldv * (size_t)(m + 1))) return DEV_ERR_DEVICE_ALLOC;
   }
   if (!part_ensure()) return DEV_ERR_DEVICE_ALLOC;
+  if (!fold_buf.p) {  // no slot of it carries a tag (tags start at 1)
+    const size_t bytes = step_fold_bytes();
+    if (fold_buf.ensure(bytes)) return DEV_ERR_DEVICE_ALLOC;
+    if (cudaMemsetAsync(fold_buf.p, 0, bytes, stream) != cudaSuccess) return DEV_ERR_UNKNOWN;
+  }
   return 0;
 }
 
@@ -2042,6 +2047,7 @@ ArnoldiArgs lace_gpu_ctx::arnoldi_args(int m, bool adjoint) {
   a.q = vec_q.p;
   a.q_f32 = vtype() != VType::F64 ? 1 : 0;
   a.partials = (double *)part_buf.p;
+  a.fold = fold_buf.p;
   a.grid = num_sms() * 8;
   a.cy = (Cycle *)cycle_buf.p;
   a.ctrl = ctrl();
@@ -2204,9 +2210,6 @@ int lace_gpu_ctx::fgmres(const double *b, double *x, int m, int restart_max, int
     LCHK(cudaMemcpyAsync(&cy->rtol, &hs.rtol, 8, cudaMemcpyHostToDevice, stream));
     int zero = 0;
     LCHK(cudaMemcpyAsync(&a.ctrl->status, &zero, 4, cudaMemcpyHostToDevice, stream));
-    // grid-barrier arrivals of the one-kernel Gram-Schmidt step (left
-    // non-zero only by a step that gave up a wait)
-    LCHK(cudaMemsetAsync(&a.ctrl->block_count[3], 0, 4, stream));
   }
   const auto key = std::make_tuple(m, adjoint ? 1 : 0, opt.trsv_mode, rows_per_lane,
                                    opt.jacobi_sweeps, (int)vtype(), opt.monitor_orthog, lanes, method,
@@ -2367,12 +2370,11 @@ extern "C" int lace_gpu_time_arnoldi_step(lace_gpu_ctx *c, int method, int j, in
   a.mgs_restarted = 1;
   a.mgs_reorth = 0;
   // the replays must neither stop nor skip: no convergence (tolerance 0),
-  // not done, barrier arrivals cleared
+  // not done
   const double zero = 0.0;
   LCHK(cudaMemcpyAsync(&a.ctrl->rtol_abs, &zero, 8, cudaMemcpyHostToDevice, c->stream));
   LCHK(cudaMemsetAsync(&a.ctrl->done, 0, 4, c->stream));
   LCHK(cudaMemsetAsync(&a.ctrl->status, 0, 4, c->stream));
-  LCHK(cudaMemsetAsync(&a.ctrl->block_count[3], 0, 4, c->stream));
   // the unsolved marks go to two scratch vectors (same element types, same
   // traffic), so that the basis and Z stay as the solve left them
   void *mt = c->vec_t2.p, *mz = c->vec_r.p;

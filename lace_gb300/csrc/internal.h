@@ -44,9 +44,6 @@ struct Cycle {
   double hinv;
   int reorth;
   int nreorth;  // steps of the cycle that reorthogonalised
-  // rows 0..j+1 of w after the step's update, published by the blocks that
-  // own them (the one-kernel Householder step)
-  double wtop[kLdT];
   // the Gram matrix V^T V of the reflectors (column-major, diagonal 1): its
   // column j+1 is V^T v_{j+1}, which step j forms for T anyway; the
   // double-float one-kernel step takes V^T w over rows > j from it
@@ -121,6 +118,7 @@ struct ArnoldiArgs {
   void *q = nullptr;     // next Krylov vector (float when q_f32, else double)
   int q_f32 = 0;
   double *partials = nullptr;  // grid-reduction scratch
+  void *fold = nullptr;        // tagged slots of the one-kernel steps (krylov_tile.cuh)
   int grid = 0;          // blocks of the reducing kernels
   Cycle *cy = nullptr;
   Control *ctrl = nullptr;
@@ -156,6 +154,7 @@ void launch_xupdate(cudaStream_t s, const ArnoldiArgs &a, double *x);
 // for shared memory), 2 when the cooperative launch failed, 0 on success
 // mark_t/mark_z (both or neither): where the unsolved marks go instead of
 // the next step's solve outputs (a measurement's replays must keep Z intact)
+size_t step_fold_bytes();  // of ArnoldiArgs::fold
 int launch_hh_step(cudaStream_t s, const ArnoldiArgs &a, int j, void *mark_t = nullptr, void *mark_z = nullptr);
 
 // ------------------------------------ FGMRES, modified Gram-Schmidt Arnoldi

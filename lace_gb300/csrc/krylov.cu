@@ -12,7 +12,7 @@
 //   pass C : v_{j+1} and q = P_0...P_{j+1} e_{j+1} (LACE :519-617) in one read
 //   x update (end of cycle): small least-squares solve + x += Z y (:721-744)
 // k_hh_step runs passes A, B and C of a step as one cooperative kernel (w in
-// shared memory, two grid reductions) where the operator is CSR and w fits;
+// shared memory, two grid sums) where the operator is CSR and w fits;
 // the separate passes serve the rest (BCSR, the adjoint, large n).
 // Every kernel returns at once when Control::done is set, so a whole cycle can
 // be launched (or replayed from a CUDA graph) without host round trips.
@@ -309,21 +309,6 @@ __global__ void __launch_bounds__(kTPB) k_cycle_init(int n, const double *__rest
   }
 }
 
-// sum_k V[k][i] c[k] over k < ncols: eight independent loads in flight
-__device__ __forceinline__ double vcomb8(const double *__restrict__ V, size_t ldv, int i, int ncols,
-                                         const double *c) {
-  double a[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-  int k = 0;
-  for (; k + 8 <= ncols; k += 8) {
-#pragma unroll
-    for (int u = 0; u < 8; ++u) a[u] = fma(V[(size_t)(k + u) * ldv + i], c[k + u], a[u]);
-  }
-#pragma unroll
-  for (int u = 0; u < 8; ++u)
-    if (k + u < ncols) a[u] = fma(V[(size_t)(k + u) * ldv + i], c[k + u], a[u]);
-  return ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
-}
-
 
 // rows i, i+1 (i even): sum_k Vf[k][i..i+1] c[k] in FP32 from the FP32 copy
 // of the reflectors, for vectors that only feed the FP32 preconditioner
@@ -343,29 +328,6 @@ __device__ __forceinline__ float2 vcomb8x2f(const float *__restrict__ Vf, size_t
       }
   }
   return make_float2((a[0].x + a[1].x) + (a[2].x + a[3].x), (a[0].y + a[1].y) + (a[2].y + a[3].y));
-}
-
-// rows i, i+1 (i even, i+1 < n): sum_k V[k][i..i+1] c[k] over k < ncols with
-// 16-byte loads, a batch of eight columns in flight before any use
-__device__ __forceinline__ double2 vcomb8x2(const double *__restrict__ V, size_t ldv, int i, int ncols,
-                                           const double *c) {
-  // two accumulators per row: the FP64 unit is the scarce one, so few
-  // closing additions matter more than a short dependency chain
-  double2 a[2] = {{0.0, 0.0}, {0.0, 0.0}};
-  for (int k = 0; k < ncols; k += 8) {
-    // a partial batch skips its missing columns
-    double2 v[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u)
-      if (k + u < ncols) v[u] = __ldg(reinterpret_cast<const double2 *>(V + (size_t)(k + u) * ldv + i));
-#pragma unroll
-    for (int u = 0; u < 8; ++u)
-      if (k + u < ncols) {
-        a[u & 1].x = fma(v[u].x, c[k + u], a[u & 1].x);
-        a[u & 1].y = fma(v[u].y, c[k + u], a[u & 1].y);
-      }
-  }
-  return make_double2(a[0].x + a[1].x, a[0].y + a[1].y);
 }
 
 // ------------------------------------------------------------- pass A
@@ -615,8 +577,8 @@ __global__ void __launch_bounds__(kTPB) k_passC(int n, double *__restrict__ V, f
 // Passes A, B and C of step j in one cooperative launch of one block per SM:
 // block b keeps rows [b*RB, (b+1)*RB) of w in shared memory through the step,
 // the two sets of dot products (V^T w, then V^T w over rows > j with ||w||^2)
-// are grid reductions (block partials, grid barrier, a fold every block
-// performs in the same order), and the small-matrix work of pass B's last
+// are grid sums (tagged block partials that every block reads and adds in the
+// same order), and the small-matrix work of pass B's last
 // block (new reflector, T column, c = T rho) is done by every block
 // identically, so pass C's combination follows without another barrier.
 // The formulas and summation orders are the passes' own.
@@ -631,109 +593,12 @@ struct HHStep {
   float *Vf;
   size_t ldv;
   void *q;
-  double *partials;  // 2 phases x kLdT x gridDim.x
+  FoldSlots fold;
   Cycle *cy;
   Control *ctrl;
   int m;
   Prefill pf;
 };
-
-// block partial sums sacc[k] = sum over this block's rows i > lo of
-// V[k][i] w[i], k < jp1: up to 32 columns as (column, row group) pairs over
-// the 32 warps, more as up to five columns per warp; lanes walk rows
-__device__ __forceinline__ void hh_block_dots(const double *__restrict__ V, size_t ldv, int jp1, int r0, int r1,
-                                              int lo, const double *sw, double *swarp, double *sacc) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int nsl = r1 > r0 ? (r1 - r0 + 31) >> 5 : 0;
-  if (jp1 <= 32) {
-    const int G = 32 / jp1;
-    double acc = 0.0;
-    if (wid < G * jp1) {
-      // a warp streams its column over 1/G of the rows: eight rows per lane
-      // in flight (one block per SM has few warps to hide the latency)
-      const int k = wid % jp1, g = wid / jp1;
-      const double *Vk = V + (size_t)k * ldv + r0;
-      for (int sl0 = g; sl0 < nsl; sl0 += 8 * G) {
-        double v[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const int t = 32 * (sl0 + u * G) + lane;
-          v[u] = (sl0 + u * G < nsl && r0 + t < r1) ? Vk[t] : 0.0;
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const int t = 32 * (sl0 + u * G) + lane;
-          const int i = r0 + t;
-          acc = fma(v[u], (sl0 + u * G < nsl && i < r1 && i > lo) ? sw[t] : 0.0, acc);
-        }
-      }
-      acc = warp_sum(acc);
-    }
-    if (lane == 0) swarp[wid] = acc;
-    __syncthreads();
-    if (threadIdx.x < jp1) {
-      double t = 0.0;
-      for (int g = 0; g < G; ++g) t += swarp[g * jp1 + threadIdx.x];
-      sacc[threadIdx.x] = t;
-    }
-  } else {
-    double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    for (int sl0 = 0; sl0 < nsl; sl0 += 4) {
-      // four rows per lane for each of the warp's columns in flight
-      double wv[4];
-      int ii[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int t = 32 * (sl0 + u) + lane;
-        const int i = r0 + t;
-        const bool ok = sl0 + u < nsl && i < r1 && i > lo;
-        wv[u] = ok ? sw[t] : 0.0;
-        ii[u] = ok ? i : r0;
-      }
-#pragma unroll
-      for (int c = 0; c < 5; ++c) {
-        const int k = wid + 32 * c;
-        if (32 * c < jp1 && k < jp1) {
-          double v[4];
-#pragma unroll
-          for (int u = 0; u < 4; ++u) v[u] = V[(size_t)k * ldv + ii[u]];
-#pragma unroll
-          for (int u = 0; u < 4; ++u) acc[c] = fma(v[u], wv[u], acc[c]);
-        }
-      }
-    }
-#pragma unroll
-    for (int c = 0; c < 5; ++c) {
-      const int k = wid + 32 * c;
-      if (32 * c < jp1) {  // warp-uniform
-        const double v = warp_sum(acc[c]);
-        if (lane == 0 && k < jp1) swarp[k] = v;
-      }
-    }
-    __syncthreads();
-    for (int k = threadIdx.x; k < jp1; k += blockDim.x) sacc[k] = swarp[k];
-  }
-  __syncthreads();
-}
-
-// sres[k] = sum over the grid of the blocks' sacc[k], k < nv, the same in
-// every block (warp w folds k = w, w+32, ...; lanes stride over the blocks)
-__device__ __forceinline__ bool hh_grid_fold(const double *sacc, int nv, double *partials, int &phase,
-                                             Control *ctrl, double *sres, int cap = kLdT) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int G = gridDim.x;
-  double *P = partials + (size_t)phase * cap * G;
-  for (int k = threadIdx.x; k < nv; k += blockDim.x) P[(size_t)k * G + blockIdx.x] = sacc[k];
-  if (!grid_barrier(ctrl)) return false;
-  for (int k = wid; k < nv; k += (int)(blockDim.x >> 5)) {
-    double t = strided_sum(P + (size_t)k * G, 1, lane, 32, G);
-    t = warp_sum(t);
-    if (lane == 0) sres[k] = t;
-  }
-  __syncthreads();
-  phase ^= 1;
-  return true;
-}
 
 template <typename ZT, typename QT>
 __global__ void __launch_bounds__(kHHTPB, 1) k_hh_step(HHStep a, int j) {
@@ -741,18 +606,20 @@ __global__ void __launch_bounds__(kHHTPB, 1) k_hh_step(HHStep a, int j) {
   constexpr bool kF32 = sizeof(QT) == 4;
   extern __shared__ double sw[];
   __shared__ double swarp[5 * 32];
-  __shared__ double sacc[kLdT + 1], sres[kLdT + 1];
+  __shared__ double sacc[kLdT + 1], sres[2 * kLdT + 1];
   __shared__ double sy[kLdT], sd[kLdT], srho[kLdT], sc[kLdT];
   __shared__ float scf[kLdT];
   __shared__ double sbuf[kHHTPB];
   __shared__ double s_dd, s_ia, s_vjj;
+  __shared__ double stop[kLdT];  // this block's rows of w up to row j+1
   const int n = a.n, jp1 = j + 1, T = blockDim.x;
   const int r0 = blockIdx.x * a.rb, r1 = min(n, r0 + a.rb);
+  const int npub = min(n, jp1 + 1), top1 = min(r1, npub);
+  const unsigned tag = *(volatile const unsigned *)a.fold.epoch + 1;  // a fold takes a tag; the last one's is left as the epoch
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const size_t ldv = a.ldv;
   const double *__restrict__ V = a.V;
   Cycle *cy = a.cy;
-  int phase = 0;
   // ---- pass A: w = A z_j (a warp per 32-row slice), s = V^T w
   {
     const ZT *z = (const ZT *)a.z;
@@ -786,7 +653,7 @@ __global__ void __launch_bounds__(kHHTPB, 1) k_hh_step(HHStep a, int j) {
   }
   __syncthreads();
   hh_block_dots(V, ldv, jp1, r0, r1, -1, sw, swarp, sacc);
-  if (!hh_grid_fold(sacc, jp1, a.partials, phase, a.ctrl, sres)) return;
+  if (!hh_grid_fold(sacc, jp1, a.fold, tag, a.ctrl, sres)) return;
   // y = T^T s
   for (int k = threadIdx.x; k < jp1; k += T) {
     double y = 0.0;
@@ -807,15 +674,15 @@ __global__ void __launch_bounds__(kHHTPB, 1) k_hh_step(HHStep a, int j) {
       sw[i + 1 - r0] = s1;
       if (i > j) nrm = fma(s0, s0, nrm);
       if (i + 1 > j) nrm = fma(s1, s1, nrm);
-      if (i <= jp1) cy->wtop[i] = s0;
-      if (i + 1 <= jp1) cy->wtop[i + 1] = s1;
+      if (i <= jp1) stop[i - r0] = s0;
+      if (i + 1 <= jp1) stop[i + 1 - r0] = s1;
     }
     if ((r1 & 1) && r1 > r0 && threadIdx.x == 0) {  // the last row of an odd n
       const int i = r1 - 1;
       const double s0 = sw[i - r0] - vcomb8(V, ldv, i, jp1, sy);
       sw[i - r0] = s0;
       if (i > j) nrm = fma(s0, s0, nrm);
-      if (i <= jp1) cy->wtop[i] = s0;
+      if (i <= jp1) stop[i - r0] = s0;
     }
   }
   sbuf[threadIdx.x] = nrm;
@@ -831,13 +698,15 @@ __global__ void __launch_bounds__(kHHTPB, 1) k_hh_step(HHStep a, int j) {
   __syncthreads();
   if (threadIdx.x == 0) sacc[jp1] = ((swarp[0] + swarp[1]) + swarp[2]) + swarp[3];
   __syncthreads();
-  if (!hh_grid_fold(sacc, jp1 + 1, a.partials, phase, a.ctrl, sres)) return;
+  if (!hh_grid_fold(sacc, jp1 + 1, a.fold, tag + 1, a.ctrl, sres, stop, r0, top1, npub)) return;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *a.fold.epoch = tag + 1;  // every block has read it
+  const double *const wtop = sres + jp1 + 1;
   // ---- pass B's last-block work, in every block: new reflector, T column,
   // c = T_{j+1} rho (LACE :476-511)
   if (threadIdx.x == 0) {
     const double nrm2 = jp1 < n ? sres[jp1] : 0.0;
     const double wn = sqrt(nrm2);
-    const double wj1 = jp1 < n ? __ldcg(&cy->wtop[jp1]) : 0.0;
+    const double wj1 = jp1 < n ? wtop[jp1] : 0.0;
     const double dd = mysgn(wj1) * wn;
     const double alpha = sqrt(2.0 * (nrm2 + fabs(wj1) * wn));
     const double ia = alpha > 0.0 ? 1.0 / alpha : 0.0;
@@ -879,7 +748,7 @@ __global__ void __launch_bounds__(kHHTPB, 1) k_hh_step(HHStep a, int j) {
       cy->inv_alpha = s_ia;
       // Hessenberg column j: h_k = w_k (k <= j), h_{j+1} = -dd (LACE :658-701)
       double *sh = sbuf;
-      for (int k = 0; k <= j; ++k) sh[k] = __ldcg(&cy->wtop[k]);
+      for (int k = 0; k <= j; ++k) sh[k] = wtop[k];
       for (int k = 0; k < j; ++k) {
         const double t0 = sh[k], t1 = sh[k + 1];
         sh[k + 1] = -cy->sn[k] * t0 + cy->cs[k] * t1;
@@ -971,7 +840,7 @@ __device__ __forceinline__ void hh_block_dots_df(const float *__restrict__ Vf, c
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int nsl = r1 > r0 ? (r1 - r0 + 31) >> 5 : 0;
   if (ncols <= 32) {
-    const int G = 32 / ncols;
+    const int G = max(1, min(32 / ncols, nsl >> 3));  // as hh_block_dots
     double acc = 0.0;
     if (wid < G * ncols) {
       const int k = wid % ncols, g = wid / ncols;
@@ -1181,7 +1050,7 @@ __global__ void __launch_bounds__(kHHTPB, 1) k_hh_step_df(HHStepDF ad, int j) {
   const HHStep &a = ad.base;
   if (a.ctrl->done) return;
   extern __shared__ float2 swd[];  // this block's rows of w, then of v_{j+1}, as (hi, lo)
-  constexpr int kCap = 2 * kLdT;   // values per grid fold
+  constexpr int kCap = kFoldCap;   // values per grid fold
   __shared__ double swarp[5 * 32];
   __shared__ double sacc[kCap], sres[kCap];
   __shared__ double sd[kLdT], srho[kLdT], sc[kLdT];
@@ -1190,15 +1059,17 @@ __global__ void __launch_bounds__(kHHTPB, 1) k_hh_step_df(HHStepDF ad, int j) {
   __shared__ float scf[kLdT];
   __shared__ double sbuf[kHHTPB];
   __shared__ double s_dd, s_ia, s_vjj;
+  __shared__ double stop[kLdT];  // this block's rows of w up to row j+1
   const int n = a.n, jp1 = j + 1, T = blockDim.x, nw = T >> 5;
   const int r0 = blockIdx.x * a.rb, r1 = min(n, r0 + a.rb);
+  const int npub = min(n, jp1 + 1), top1 = min(r1, npub);
+  const unsigned tag = *(volatile const unsigned *)a.fold.epoch + 1;  // a fold takes a tag; the last one's is left as the epoch
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const size_t ldv = a.ldv;
   const float *__restrict__ Vf = a.Vf;
   const float *__restrict__ Vlo = ad.Vlo;
   Cycle *cy = a.cy;
   const int G = gridDim.x;
-  int phase = 0;
   // g's block partials from the previous step, folded with s below
   for (int k = threadIdx.x; k < j; k += T) sacc[jp1 + k] = __ldcg(&ad.carry[(size_t)k * G + blockIdx.x]);
   // ---- pass A: w = A z_j in pair arithmetic (the operator's values as
@@ -1236,7 +1107,7 @@ __global__ void __launch_bounds__(kHHTPB, 1) k_hh_step_df(HHStepDF ad, int j) {
   }
   __syncthreads();
   hh_block_dots_df(Vf, Vlo, ldv, jp1, r0, r1, -1, DfShared{swd}, swarp, sacc);
-  if (!hh_grid_fold(sacc, jp1 + j, a.partials, phase, a.ctrl, sres, kCap)) return;
+  if (!hh_grid_fold(sacc, jp1 + j, a.fold, tag, a.ctrl, sres)) return;
   // T(:, j) = [-2 T_j g ; 2] and G(:, j) = [g ; 1] (a warp per entry)
   for (int k = wid; k <= j; k += nw) {
     double t = 0.0;
@@ -1284,8 +1155,8 @@ __global__ void __launch_bounds__(kHHTPB, 1) k_hh_step_df(HHStepDF ad, int j) {
       swd[i + 1 - r0] = s1;
       if (i > j) df_mac(s0.x, s0.y, s0.x, s0.y, nh, nl);
       if (i + 1 > j) df_mac(s1.x, s1.y, s1.x, s1.y, nh, nl);
-      if (i <= jp1) cy->wtop[i] = df_join(s0);
-      if (i + 1 <= jp1) cy->wtop[i + 1] = df_join(s1);
+      if (i <= jp1) stop[i - r0] = df_join(s0);
+      if (i + 1 <= jp1) stop[i + 1 - r0] = df_join(s1);
     }
     if ((r1 & 1) && r1 > r0 && threadIdx.x == 0) {  // the last row of an odd n
       const int i = r1 - 1;
@@ -1293,7 +1164,7 @@ __global__ void __launch_bounds__(kHHTPB, 1) k_hh_step_df(HHStepDF ad, int j) {
       const float2 s0 = df_add(swd[i - r0], make_float2(-c.x, -c.y));
       swd[i - r0] = s0;
       if (i > j) df_mac(s0.x, s0.y, s0.x, s0.y, nh, nl);
-      if (i <= jp1) cy->wtop[i] = df_join(s0);
+      if (i <= jp1) stop[i - r0] = df_join(s0);
     }
     nrm = to_f64(nh) + to_f64(nl);
   }
@@ -1309,7 +1180,9 @@ __global__ void __launch_bounds__(kHHTPB, 1) k_hh_step_df(HHStepDF ad, int j) {
   __syncthreads();
   if (threadIdx.x == 0) sacc[0] = ((swarp[0] + swarp[1]) + swarp[2]) + swarp[3];
   __syncthreads();
-  if (!hh_grid_fold(sacc, 1, a.partials, phase, a.ctrl, sres, kCap)) return;
+  if (!hh_grid_fold(sacc, 1, a.fold, tag + 1, a.ctrl, sres, stop, r0, top1, npub)) return;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *a.fold.epoch = tag + 1;  // every block has read it
+  const double *const wtop = sres + 1;
   const double nrm2 = jp1 < n ? sres[0] : 0.0;
   // V^T w over rows > j after the update, without a pass over V:
   // s - G y over all rows, less the rows <= j that their owners published
@@ -1319,13 +1192,13 @@ __global__ void __launch_bounds__(kHHTPB, 1) k_hh_step_df(HHStepDF ad, int j) {
       const double gkl = l == j ? sg[k] : (k == j ? sg[l] : cy->G[k + l * kLdT]);
       t = fma(gkl, sy[l], t);
     }
-    for (int i = k + lane; i <= j; i += 32) t = fma(a.V[(size_t)k * ldv + i], __ldcg(&cy->wtop[i]), t);
+    for (int i = k + lane; i <= j; i += 32) t = fma(a.V[(size_t)k * ldv + i], wtop[i], t);
     t = warp_sum(t);
     if (lane == 0) s2[k] = ss[k] - t;
   }
   if (threadIdx.x == 0) {
     const double wn = sqrt(nrm2);
-    const double wj1 = jp1 < n ? __ldcg(&cy->wtop[jp1]) : 0.0;
+    const double wj1 = jp1 < n ? wtop[jp1] : 0.0;
     const double dd = mysgn(wj1) * wn;
     const double alpha = sqrt(2.0 * (nrm2 + fabs(wj1) * wn));
     const double ia = alpha > 0.0 ? 1.0 / alpha : 0.0;
@@ -1414,7 +1287,7 @@ __global__ void __launch_bounds__(kHHTPB, 1) k_hh_step_df(HHStepDF ad, int j) {
   if (blockIdx.x == G - 1) {
     double *sh = sbuf, *scs = sbuf + 256, *ssn = sbuf + 512;
     if (wid == 0) {
-      for (int k = lane; k <= j; k += 32) sh[k] = __ldcg(&cy->wtop[k]);
+      for (int k = lane; k <= j; k += 32) sh[k] = wtop[k];
       for (int k = lane; k < j; k += 32) {
         scs[k] = cy->cs[k];
         ssn[k] = cy->sn[k];
@@ -1661,15 +1534,16 @@ static int hh_step_t(cudaStream_t s, const ArnoldiArgs &a, int j, void *mark_t, 
   if (G == 0) return 1;
   HHStep p;
   p.n = a.n;
-  p.rb = ((a.n + G - 1) / G + 31) / 32 * 32;
-  if ((size_t)p.rb * 8 > (size_t)kHHSmemMax || (size_t)G * kLdT * 2 > (size_t)a.grid * kLdT) return 1;
+  p.rb = step_rows(a.n, G);
+  if ((size_t)p.rb * 8 > (size_t)kHHSmemMax) return 1;
+  const int blocks = (a.n + p.rb - 1) / p.rb;
   p.op = opview(a);
   p.z = (const char *)a.Z + (size_t)j * a.ldz * sizeof(ZT);
   p.V = a.V;
   p.Vf = a.Vf;
   p.ldv = a.ldv;
   p.q = a.q;
-  p.partials = a.partials;
+  p.fold = fold_slots(a.fold);
   p.cy = a.cy;
   p.ctrl = a.ctrl;
   p.m = a.m;
@@ -1679,7 +1553,7 @@ static int hh_step_t(cudaStream_t s, const ArnoldiArgs &a, int j, void *mark_t, 
     p.pf.z = mark_z;
   }
   void *args[] = {&p, &j};
-  if (cudaLaunchCooperativeKernel((const void *)k_hh_step<ZT, QT>, dim3(G), dim3(kHHTPB), args,
+  if (cudaLaunchCooperativeKernel((const void *)k_hh_step<ZT, QT>, dim3(blocks), dim3(kHHTPB), args,
                                   (size_t)p.rb * 8, s) != cudaSuccess) {
     cudaGetLastError();
     return 2;
@@ -1703,17 +1577,18 @@ static int hh_step_df(cudaStream_t s, const ArnoldiArgs &a, int j, void *mark_t,
   HHStepDF pd;
   HHStep &p = pd.base;
   p.n = a.n;
-  p.rb = ((a.n + G - 1) / G + 31) / 32 * 32;
-  // two phases of 2 kLdT fold values per block, then the carried partials,
-  // in the partials buffer
+  p.rb = step_rows(a.n, G);
+  // the carried partials sit in the partials buffer, past what the
+  // orthogonality monitor uses of it between two steps
   if ((size_t)p.rb * 8 > (size_t)kHHSmemMax || (size_t)G * kLdT * 5 > (size_t)a.grid * kLdT) return 1;
+  const int blocks = (a.n + p.rb - 1) / p.rb;
   p.op = opview(a);
   p.z = (const char *)a.Z + (size_t)j * a.ldz * sizeof(float);
   p.V = a.V;
   p.Vf = a.Vf;
   p.ldv = a.ldv;
   p.q = a.q;
-  p.partials = a.partials;
+  p.fold = fold_slots(a.fold);
   p.cy = a.cy;
   p.ctrl = a.ctrl;
   p.m = a.m;
@@ -1726,13 +1601,15 @@ static int hh_step_df(cudaStream_t s, const ArnoldiArgs &a, int j, void *mark_t,
   pd.carry = a.partials + (size_t)4 * kLdT * G;
   pd.sell_pair = a.sell_pair;
   void *args[] = {&pd, &j};
-  if (cudaLaunchCooperativeKernel((const void *)k_hh_step_df, dim3(G), dim3(kHHTPB), args, (size_t)p.rb * 8, s) !=
+  if (cudaLaunchCooperativeKernel((const void *)k_hh_step_df, dim3(blocks), dim3(kHHTPB), args, (size_t)p.rb * 8, s) !=
       cudaSuccess) {
     cudaGetLastError();
     return 2;
   }
   return 0;
 }
+
+size_t step_fold_bytes() { return fold_bytes(num_sms()); }
 
 int launch_hh_step(cudaStream_t s, const ArnoldiArgs &a, int j, void *mark_t, void *mark_z) {
   if (a.bs || !a.sell_ptr) return 1;

@@ -204,6 +204,45 @@ __device__ void mgs_finish(int j, int m, int restarted, Cycle *cy, Control *ctrl
   }
 }
 
+// The same for the one-kernel steps, by one thread: the column in sh (its
+// rotated form left there), the rotations so far in scs and ssn, so that its
+// serial chain reads shared memory only; hj1 is h_{j+1}.
+__device__ void mgs_finish_staged(int j, int m, double hj1, double *sh, const double *scs, const double *ssn, Cycle *cy,
+                                  Control *ctrl) {
+  double g0 = cy->g[j], g1 = cy->g[j + 1];  // on their way during the chain
+  const double tol = ctrl->rtol_abs;
+  sh[j + 1] = hj1;
+  for (int k = 0; k < j; ++k) {  // :406-415
+    const double delta = sh[k], next = sh[k + 1];
+    sh[k] = scs[k] * delta - ssn[k] * next;
+    sh[k + 1] = ssn[k] * delta + scs[k] * next;
+  }
+  const double gamma = sqrt(sh[j] * sh[j] + hj1 * hj1);  // :417-420
+  if (gamma > 0.0) {                                     // :421-432
+    const double c = sh[j] / gamma, s = -hj1 / gamma;
+    cy->cs[j] = c;
+    cy->sn[j] = s;
+    sh[j] = c * sh[j] - s * hj1;
+    sh[j + 1] = 0.0;
+    const double delta = g0;
+    g0 = c * delta - s * g1;
+    g1 = s * delta + c * g1;
+    cy->g[j] = g0;
+    cy->g[j + 1] = g1;
+  }
+  const double resid = fabs(g1);
+  cy->hist[j] = resid;
+  ctrl->resid = resid;
+  const bool conv = resid < tol;
+  const bool finite = isfinite(g1);
+  if (conv || j == m - 1 || !finite) {  // as mgs_finish
+    ctrl->nsteps = j + 1;
+    ctrl->converged = conv ? 1 : 0;
+    if (!finite) ctrl->status |= kStatusBreakdown;
+    ctrl->done = 1;
+  }
+}
+
 // u -= c_j v_j, h_{j+1} = ||u|| (:329-333).  Pass 0: the Brown/Hindmarsh
 // test (:336-338) decides the second pass (cond set to 1, the rotations
 // wait for it); otherwise, and after pass 1 (:360), the rotations and the
@@ -318,10 +357,10 @@ __global__ void __launch_bounds__(kTPB) k_mgs_xupdate(int n, const ZT *__restric
 // The whole Arnoldi step after the solves (operator, both Gram-Schmidt
 // passes, rotations, the next basis vector) in one cooperative launch of
 // one block per SM: block b keeps rows [b*RB, (b+1)*RB) of u in shared
-// memory, and each Gram-Schmidt sum is a block sum, a grid barrier and a
-// fold of the blocks' partial sums that every block performs in the same
-// order, so every block holds the same coefficient.  u never leaves the SM;
-// a sum costs one barrier instead of a kernel boundary.
+// memory, and each Gram-Schmidt sum is a block sum and a fold of the blocks'
+// tagged partial sums that every block performs in the same order, so every
+// block holds the same coefficient.  u never leaves the SM;
+// a sum costs one trip through L2 instead of a kernel boundary.
 constexpr int kStepTPB = 1024;
 constexpr int kStepSmemMax = 200 * 1024;  // rows of u per block: at most 25,600 (plus 16 KB static)
 
@@ -329,16 +368,16 @@ constexpr int kStepSmemMax = 200 * 1024;  // rows of u per block: at most 25,600
 // this part's scarce resource, so both reductions stage the values in
 // shared memory and let few warps add them (a butterfly in every warp would
 // cost five FP64 adds per warp): the block's threads' values are summed by
-// four warps (one per SM sub-partition) and the four results in order; after
-// the barrier one warp folds the grid's partial sums.  Fixed orders: every
-// block computes the same value.  partials: 4 x gridDim.x doubles, two
-// phases so that a block may run ahead into the next sum while others still
-// fold this one.  sbuf: NV x blockDim.x doubles; sred: 8 * NV + NV doubles.
+// four warps (one per SM sub-partition) and the four results in order; then a
+// warp per value adds the grid's tagged partial sums (krylov_tile.cuh).  Fixed
+// orders: every block computes the same value.  sbuf: NV x blockDim.x doubles;
+// sred: 8 * NV + NV doubles.
 template <int NV>
-__device__ __forceinline__ bool grid_sum(double (&v)[NV], double *partials, int &phase, Control *ctrl,
-                                         double *sbuf, double *sred) {
+__device__ __forceinline__ bool grid_sum(double (&v)[NV], const FoldSlots &f, unsigned &tag, Control *ctrl, double *sbuf,
+                                         double *sred) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int T = blockDim.x, G = gridDim.x;
+  ulonglong2 *P = f.slot + (size_t)(tag & 1) * kFoldCap * G;
 #pragma unroll
   for (int q = 0; q < NV; ++q) sbuf[q * T + threadIdx.x] = v[q];
   __syncthreads();
@@ -354,23 +393,18 @@ __device__ __forceinline__ bool grid_sum(double (&v)[NV], double *partials, int 
   }
   __syncthreads();
   if (threadIdx.x < NV)
-    partials[(size_t)(phase * 2 + threadIdx.x) * G + blockIdx.x] =
-        ((sred[threadIdx.x * 8] + sred[threadIdx.x * 8 + 1]) + sred[threadIdx.x * 8 + 2]) + sred[threadIdx.x * 8 + 3];
-  if (!grid_barrier(ctrl)) return false;
-  if (wid == 0) {
-#pragma unroll
-    for (int q = 0; q < NV; ++q) {
-      double t = 0.0;
-      for (int b = lane; b < G; b += 32) t += __ldcg(partials + (size_t)(phase * 2 + q) * G + b);
-      t = warp_sum(t);
-      if (lane == 0) sred[8 * NV + q] = t;
-    }
+    tag_put(P + (size_t)threadIdx.x * G + blockIdx.x,
+            ((sred[threadIdx.x * 8] + sred[threadIdx.x * 8 + 1]) + sred[threadIdx.x * 8 + 2]) + sred[threadIdx.x * 8 + 3],
+            tag);
+  bool ok = true;
+  if (wid < NV) {
+    const double t = warp_sum(tag_lane_sum(P + (size_t)wid * G, G, tag, ctrl, ok));
+    if (lane == 0) sred[8 * NV + wid] = t;
   }
-  __syncthreads();
+  if (!__syncthreads_and(ok)) return false;
 #pragma unroll
   for (int q = 0; q < NV; ++q) v[q] = sred[8 * NV + q];
-  __syncthreads();
-  phase ^= 1;
+  ++tag;
   return true;
 }
 
@@ -380,12 +414,63 @@ struct MgsStep {
   const void *z;
   double *V;
   size_t ldv;
-  double *partials;
+  FoldSlots fold;
   Cycle *cy;
   Control *ctrl;
   int m, restarted, reorth;
   Prefill pf;
 };
+
+// what every thread of a one-kernel step needs of the step's scalars, formed by
+// one of them (a square root or a division by all warps holds the SM's FP64
+// unit for microseconds)
+struct MgsScalars {
+  double normav, hn, inv;  // ||A z||, ||u||, 1 / h_{j+1} (0 after a breakdown)
+  int again;
+};
+__device__ __forceinline__ void mgs_scalars(const MgsStep &a, double hn2, MgsScalars &s) {
+  const double hn = sqrt(hn2), brk = a.restarted ? 0.0 : DBL_EPSILON;
+  s.hn = hn;
+  s.inv = fabs(hn) > brk ? 1.0 / hn : 0.0;
+  const double hr = (s.normav + 0.001 * hn) - s.normav;  // :336-338
+  s.again = ((a.reorth == 0 && hr <= 4.9406564584124654e-324) || a.reorth == 2) ? 1 : 0;
+}
+// the column, the rotations and the convergence test, in the last block (the
+// fewest rows) once its rows of v_{j+1} are out; again: whether the step
+// reorthogonalised
+__device__ __forceinline__ void mgs_column(const MgsStep &a, int j, int again, const MgsScalars &s, double *sh,
+                                           const double *scs, const double *ssn) {
+  if (blockIdx.x != gridDim.x - 1) return;
+  if (threadIdx.x == 0) {
+    a.cy->nreorth += again;
+    mgs_finish_staged(j, a.m, s.hn, sh, scs, ssn, a.cy, a.ctrl);
+  }
+  __syncthreads();
+  double *R = a.cy->R + (size_t)j * kLdT;
+  for (int k = threadIdx.x; k <= j + 1; k += blockDim.x) R[k] = sh[k];
+}
+
+// v_{j+1} = u / h_{j+1} (zero after a breakdown) for this block's rows, the
+// next solves' outputs marked
+__device__ __forceinline__ void mgs_next_rows(const MgsStep &a, int j, double inv, const double *su) {
+  const int r0 = blockIdx.x * a.rb, r1 = min(a.n, r0 + a.rb), T = blockDim.x;
+  const int p0 = r0 >> 1, p1 = r1 >> 1;
+  const bool tail = (r1 & 1) && r1 > r0 && threadIdx.x == 0;
+  const double2 *su2 = reinterpret_cast<const double2 *>(su);
+  double *vn = a.V + (size_t)(j + 1) * a.ldv;
+  double2 *vn2 = reinterpret_cast<double2 *>(vn);
+#pragma unroll 4
+  for (int p = p0 + threadIdx.x; p < p1; p += T) {
+    const double2 u = su2[p - p0];
+    vn2[p] = inv == 0.0 ? make_double2(0.0, 0.0) : make_double2(u.x * inv, u.y * inv);
+    prefill_row(a.pf, 2 * p);
+    prefill_row(a.pf, 2 * p + 1);
+  }
+  if (tail) {
+    vn[r1 - 1] = inv == 0.0 ? 0.0 : su[r1 - 1 - r0] * inv;
+    prefill_row(a.pf, r1 - 1);
+  }
+}
 
 template <typename ZT>
 __global__ void __launch_bounds__(kStepTPB, 1) k_mgs_step(MgsStep a, int j) {
@@ -393,11 +478,16 @@ __global__ void __launch_bounds__(kStepTPB, 1) k_mgs_step(MgsStep a, int j) {
   extern __shared__ double su[];
   __shared__ double sbuf[2 * kStepTPB];
   __shared__ double sred[8 * 2 + 2];
-  __shared__ double sh[kLdT + 1];
+  __shared__ double sh[kLdT + 1], scs[kLdT], ssn[kLdT];
+  __shared__ MgsScalars sc;
   const int r0 = blockIdx.x * a.rb, r1 = min(a.n, r0 + a.rb);
   const int T = blockDim.x;
+  for (int k = threadIdx.x; k < j; k += T) {
+    scs[k] = a.cy->cs[k];
+    ssn[k] = a.cy->sn[k];
+  }
   const ZT *z = (const ZT *)a.z;
-  int phase = 0;
+  unsigned tag = *(volatile const unsigned *)a.fold.epoch + 1;  // one a sum; the last one's is left as the epoch
   // u = A z_j for this block's rows (a warp per 32-row slice), ||u||^2, v_0 . u
   double acc[2] = {0.0, 0.0};
   {
@@ -432,13 +522,14 @@ __global__ void __launch_bounds__(kStepTPB, 1) k_mgs_step(MgsStep a, int j) {
       }
     }
   }
-  if (!grid_sum<2>(acc, a.partials, phase, a.ctrl, sbuf, sred)) return;
-  const double normav = sqrt(acc[0]);
-  if (threadIdx.x == 0) sh[0] = acc[1];
+  if (!grid_sum<2>(acc, a.fold, tag, a.ctrl, sbuf, sred)) return;
+  if (threadIdx.x == 0) {
+    sh[0] = acc[1];
+    sc.normav = sqrt(acc[0]);
+  }
   __syncthreads();
   // Gram-Schmidt passes: sums k = 1..j+1 (the last one the norm); pass 1
   // (the second pass) only when the Brown/Hindmarsh test asks
-  double hn = 0.0;
   int again = 0;
   // the vector loops walk row pairs (16-byte loads, four pairs per thread in
   // flight: one 8-byte load per thread would keep too few bytes in flight to
@@ -459,7 +550,7 @@ __global__ void __launch_bounds__(kStepTPB, 1) k_mgs_step(MgsStep a, int j) {
         d[0] = fma(v.y, u.y, d[0]);
       }
       if (tail) d[0] = fma(a.V[r1 - 1], su[r1 - 1 - r0], d[0]);
-      if (!grid_sum<1>(d, a.partials, phase, a.ctrl, sbuf, sred)) return;
+      if (!grid_sum<1>(d, a.fold, tag, a.ctrl, sbuf, sred)) return;
       c = d[0];
       if (threadIdx.x == 0) sh[0] += c;
     }
@@ -502,76 +593,214 @@ __global__ void __launch_bounds__(kStepTPB, 1) k_mgs_step(MgsStep a, int j) {
           d[0] = fma(ui, ui, d[0]);
         }
       }
-      if (!grid_sum<1>(d, a.partials, phase, a.ctrl, sbuf, sred)) return;
+      if (!grid_sum<1>(d, a.fold, tag, a.ctrl, sbuf, sred)) return;
       if (k <= j) {
         c = d[0];
         if (threadIdx.x == 0) sh[k] = pass ? sh[k] + c : c;
-      } else {
-        hn = sqrt(d[0]);
+      } else if (threadIdx.x == 0) {
+        mgs_scalars(a, d[0], sc);
       }
       __syncthreads();
     }
     if (pass) break;
-    const double hr = (normav + 0.001 * hn) - normav;  // :336-338
-    again = ((a.reorth == 0 && hr <= 4.9406564584124654e-324) || a.reorth == 2) ? 1 : 0;
+    again = sc.again;
     if (!again) break;
   }
-  // block 0: the column, the rotations and the convergence test
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    Cycle *cy = a.cy;
-    for (int k = 0; k <= j; ++k) cy->h[k] = sh[k];
-    cy->h[j + 1] = hn;
-    cy->normav = normav;
-    cy->reorth = again;
-    cy->nreorth += again;
-    mgs_finish(j, a.m, a.restarted, cy, a.ctrl);
+  if (blockIdx.x == 0 && threadIdx.x == 0) *a.fold.epoch = tag - 1;  // every block has read it
+  mgs_next_rows(a, j, sc.inv, su);
+  mgs_column(a, j, again, sc, sh, scs, ssn);
+}
+
+// The same step with two sums over the grid instead of j + 2.  The
+// coefficients of modified Gram-Schmidt, h_k = v_k . (u - sum_{i<k} h_i v_i),
+// are h = (I + L)^{-1} V^T u with L the strictly lower part of V^T V, so one
+// fold of V^T u, V^T v_j (L's new row) and ||u||^2 gives them all; T = (I +
+// L)^{-1} grows by the row -(V^T v_j)^T T a step.  Same rounding level as the
+// column-by-column form (L is the basis's departure from orthogonality), three
+// FP64 multiply-adds per row and column instead of two: where a sum over the
+// grid costs more than that third pass (below).  u and v_j in shared memory;
+// the second pass when the Brown/Hindmarsh test asks is one more fold of V^T u
+// and one of the norm.
+template <typename ZT>
+__global__ void __launch_bounds__(kStepTPB, 1) k_mgs_step_ls(MgsStep a, int j) {
+  if (a.ctrl->done) return;
+  extern __shared__ double su[];
+  double *sv = su + a.rb;
+  __shared__ double swarp[5 * 32], sacc[kFoldCap], sres[kFoldCap];
+  __shared__ double st[kLdT], sh[kLdT + 1], ss[kLdT], shr[kLdT];
+  __shared__ double sbuf[kStepTPB], scs[kLdT], ssn[kLdT];
+  __shared__ MgsScalars sc;
+  const int r0 = blockIdx.x * a.rb, r1 = min(a.n, r0 + a.rb), jp1 = j + 1, T = blockDim.x;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = T >> 5;
+  const ZT *z = (const ZT *)a.z;
+  double *const Tm = a.cy->T, *const Tt = a.cy->G;  // T and its transpose (lower, unit diagonal)
+  for (int k = threadIdx.x; k < j; k += T) {
+    scs[k] = a.cy->cs[k];
+    ssn[k] = a.cy->sn[k];
   }
-  // v_{j+1} = u / h_{j+1} (zero after a breakdown), the next solves' outputs marked
-  const double brk = a.restarted ? 0.0 : DBL_EPSILON;
-  const double inv = fabs(hn) > brk ? 1.0 / hn : 0.0;
-  double *vn = a.V + (size_t)(j + 1) * a.ldv;
-  double2 *vn2 = reinterpret_cast<double2 *>(vn);
+  unsigned tag = *(volatile const unsigned *)a.fold.epoch + 1;  // one a fold; the last one's is left as the epoch
+  // sum over the block of the threads' v, by four warps (few FP64 adds), valid
+  // after the call; only as many threads as there are rows have one
+  const int busy = min(T, (r1 - r0 + 127) / 128 * 128);
+  auto block_total = [&](double v, double *out) {
+    sbuf[threadIdx.x] = v;
+    __syncthreads();
+    if (wid < 4) {
+      const int quarter = busy >> 2;
+      double t = 0.0;
+      for (int k = wid * quarter + lane; k < (wid + 1) * quarter; k += 32) t += sbuf[k];
+      t = warp_sum(t);
+      if (lane == 0) swarp[wid] = t;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) *out = ((swarp[0] + swarp[1]) + swarp[2]) + swarp[3];
+    __syncthreads();
+  };
+  // u = A z_j (a warp per 32-row slice), v_j's rows beside it
+  double nrm = 0.0;
+  for (int sl = (r0 >> 5) + wid; 32 * sl < r1; sl += nw) {
+    const int i = 32 * sl + lane;
+    if (i < r1) {
+      const int len = a.op.row[i + 1] - a.op.row[i];
+      const int *cp = a.op.sell_col + a.op.sell_ptr[sl] + lane;
+      const double *vp = a.op.sell_val + (cp - a.op.sell_col);
+      double s = 0.0;
+      for (int t = 0; t < len; t += 8) {  // a 7-point row in one round of loads
+        int c[8];
+        double v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          if (t + u < len) {
+            c[u] = cp[32 * (t + u)];
+            v[u] = vp[32 * (t + u)];
+          }
+        ZT zv[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          if (t + u < len) zv[u] = z[c[u]];
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          if (t + u < len) s = fma(v[u], to_f64(zv[u]), s);
+      }
+      su[i - r0] = s;
+      sv[i - r0] = a.V[(size_t)j * a.ldv + i];
+      nrm = fma(s, s, nrm);
+    }
+  }
+  __syncthreads();
+  hh_block_dots(a.V, a.ldv, jp1, r0, r1, -1, su, swarp, sacc);
+  if (j > 0) hh_block_dots(a.V, a.ldv, j, r0, r1, -1, sv, swarp, sacc + jp1);
+  block_total(nrm, &sacc[2 * j + 1]);
+  if (!hh_grid_fold(sacc, 2 * j + 2, a.fold, tag++, a.ctrl, sres)) return;
+  // T's row j, then h = T V^T u: four threads an entry
+  const int e = threadIdx.x >> 2, part = threadIdx.x & 3;
+  auto quad = [&](double v) {
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    return v + __shfl_xor_sync(0xffffffffu, v, 2);
+  };
+  {
+    double t = 0.0;
 #pragma unroll 4
-  for (int p = p0 + threadIdx.x; p < p1; p += T) {
-    const double2 u = su2[p - p0];
-    vn2[p] = inv == 0.0 ? make_double2(0.0, 0.0) : make_double2(u.x * inv, u.y * inv);
-    prefill_row(a.pf, 2 * p);
-    prefill_row(a.pf, 2 * p + 1);
+    for (int k = e + part; k < j; k += 4) t = fma(sres[jp1 + k], Tt[e + (size_t)k * kLdT], t);
+    t = quad(t);
+    if (part == 0 && e <= j) st[e] = e < j ? -t : 1.0;
   }
-  if (tail) {
-    vn[r1 - 1] = inv == 0.0 ? 0.0 : su[r1 - 1 - r0] * inv;
-    prefill_row(a.pf, r1 - 1);
+  for (int k = threadIdx.x; k < jp1; k += T) ss[k] = sres[k];
+  if (threadIdx.x == 0) sc.normav = sqrt(sres[2 * j + 1]);
+  __syncthreads();
+  auto coefficients = [&](double *h) {
+    double t = 0.0;
+    if (e <= j) {
+#pragma unroll 4
+      for (int i = part; i <= e; i += 4) t = fma(e < j ? Tm[e + (size_t)i * kLdT] : st[i], ss[i], t);
+    }
+    t = quad(t);
+    if (part == 0 && e <= j) h[e] = t;
+    __syncthreads();
+  };
+  coefficients(sh);
+  if (blockIdx.x == 0)
+    for (int i = threadIdx.x; i <= j; i += T) {  // read by the later steps only
+      Tm[j + (size_t)i * kLdT] = st[i];
+      Tt[i + (size_t)j * kLdT] = st[i];
+    }
+  // u -= V h (a row pair per thread) and ||u||
+  const int p0 = r0 >> 1, p1 = r1 >> 1;
+  const bool tail = (r1 & 1) && r1 > r0 && threadIdx.x == 0;
+  double2 *su2 = reinterpret_cast<double2 *>(su);
+  auto update = [&](const double *h) {
+    double d = 0.0;
+    for (int p = p0 + threadIdx.x; p < p1; p += T) {
+      const double2 c = vcomb8x2(a.V, a.ldv, 2 * p, jp1, h);
+      double2 u = su2[p - p0];
+      u.x -= c.x;
+      u.y -= c.y;
+      su2[p - p0] = u;
+      d = fma(u.x, u.x, d);
+      d = fma(u.y, u.y, d);
+    }
+    if (tail) {
+      const double u = su[r1 - 1 - r0] - vcomb8(a.V, a.ldv, r1 - 1, jp1, h);
+      su[r1 - 1 - r0] = u;
+      d = fma(u, u, d);
+    }
+    block_total(d, &sacc[0]);
+    if (!hh_grid_fold(sacc, 1, a.fold, tag++, a.ctrl, sres)) return false;
+    if (threadIdx.x == 0) mgs_scalars(a, sres[0], sc);
+    __syncthreads();
+    return true;
+  };
+  if (!update(sh)) return;
+  const int again = sc.again;
+  if (again) {
+    __syncthreads();
+    hh_block_dots(a.V, a.ldv, jp1, r0, r1, -1, su, swarp, sacc);
+    if (!hh_grid_fold(sacc, jp1, a.fold, tag++, a.ctrl, sres)) return;
+    for (int k = threadIdx.x; k < jp1; k += T) ss[k] = sres[k];
+    __syncthreads();
+    coefficients(shr);
+    if (!update(shr)) return;
+    for (int k = threadIdx.x; k < jp1; k += T) sh[k] += shr[k];
+    __syncthreads();
   }
+  if (blockIdx.x == 0 && threadIdx.x == 0) *a.fold.epoch = tag - 1;  // every block has read it
+  mgs_next_rows(a, j, sc.inv, su);
+  mgs_column(a, j, again, sc, sh, scs, ssn);
 }
 
 // -------------------------------------------------------------- launchers
 
+// one block per SM when the kernel fits there with the largest shared memory
+// (0: it does not)
+static int step_blocks(const void *kernel) {
+  int per_sm = 0;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStepSmemMax) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kStepTPB, kStepSmemMax) != cudaSuccess ||
+      per_sm < 1) {
+    cudaGetLastError();
+    return 0;
+  }
+  return num_sms();
+}
+
 template <typename ZT>
 static int mgs_step_t(cudaStream_t s, const ArnoldiArgs &a, int j, void *mark_t, void *mark_z) {
-  // one block per SM when the kernel fits there with the largest shared
-  // memory (0: it does not); set once, thread-safely
-  static const int G = [] {
-    int per_sm = 0;
-    if (cudaFuncSetAttribute(k_mgs_step<ZT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStepSmemMax) !=
-            cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_mgs_step<ZT>, kStepTPB, kStepSmemMax) !=
-            cudaSuccess ||
-        per_sm < 1) {
-      cudaGetLastError();
-      return 0;
-    }
-    return num_sms();
-  }();
-  if (G == 0) return 1;
+  static const int G = step_blocks((const void *)k_mgs_step<ZT>);  // set once, thread-safely
+  static const int Gls = step_blocks((const void *)k_mgs_step_ls<ZT>);
+  // two sums over the grid where u and v_j fit shared memory (16 bytes a row:
+  // 1.9 M rows on 152 SMs), else a sum per column
+  const bool ls = Gls > 0 && (size_t)step_rows(a.n, Gls) * 16 <= (size_t)kStepSmemMax;
+  if (!ls && G == 0) return 1;
   MgsStep p;
   p.n = a.n;
-  p.rb = ((a.n + G - 1) / G + 31) / 32 * 32;
-  if ((size_t)p.rb * 8 > (size_t)kStepSmemMax) return 1;
+  p.rb = step_rows(a.n, ls ? Gls : G);
+  const size_t smem = (size_t)p.rb * (ls ? 16 : 8);
+  if (smem > (size_t)kStepSmemMax) return 1;
   p.op = opview(a);
   p.z = (const char *)a.Z + (size_t)j * a.ldz * sizeof(ZT);
   p.V = a.V;
   p.ldv = a.ldv;
-  p.partials = a.partials;
+  p.fold = fold_slots(a.fold);
   p.cy = a.cy;
   p.ctrl = a.ctrl;
   p.m = a.m;
@@ -583,8 +812,9 @@ static int mgs_step_t(cudaStream_t s, const ArnoldiArgs &a, int j, void *mark_t,
     p.pf.z = mark_z;
   }
   void *args[] = {&p, &j};
-  if (cudaLaunchCooperativeKernel((const void *)k_mgs_step<ZT>, dim3(G), dim3(kStepTPB), args,
-                                  (size_t)p.rb * 8, s) != cudaSuccess) {
+  const int blocks = (a.n + p.rb - 1) / p.rb;
+  if (cudaLaunchCooperativeKernel(ls ? (const void *)k_mgs_step_ls<ZT> : (const void *)k_mgs_step<ZT>, dim3(blocks),
+                                  dim3(kStepTPB), args, smem, s) != cudaSuccess) {
     cudaGetLastError();
     return 2;
   }

@@ -193,37 +193,233 @@ __device__ __forceinline__ void prefill_row(const Prefill &f, size_t i) {
 
 // ------------------------------------- persistent (cooperative) kernels
 
-// Grid barrier over a cooperatively launched grid (Control::block_count[3]
-// arrivals, [4] generation).  Bounded: a wait that gives up sets
-// kStatusSpinTimeout, and every block leaves at its next barrier.
-__device__ __forceinline__ bool grid_barrier(Control *ctrl) {
-  __shared__ int s_ok;
-  __threadfence();  // every thread's writes before the arrival (partial sums)
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int *count = &ctrl->block_count[3];
-    int *gen = &ctrl->block_count[4];
-    const int g = ld_acquire(gen);
-    __threadfence();
-    int ok = 1;
-    if (atomicAdd(count, 1) == (int)gridDim.x - 1) {
-      *count = 0;
-      st_release(gen, g + 1);
-    } else {
-      for (int spins = 0;; ++spins) {
-        if (ld_acquire(gen) != g) break;
-        if (spins > kMaxSpins || ((spins & 1023) == 1023 && (ld_relaxed(&ctrl->status) & kStatusSpinTimeout))) {
-          atomicOr(&ctrl->status, kStatusSpinTimeout);
-          ok = 0;
-          break;
-        }
-        if (spins > 32) __nanosleep(32);
+// Sums over a cooperatively launched grid without a barrier: every block
+// stores its partial sums with a tag, and every block reads all of them until
+// the tags are there, so a sum costs one trip through L2 and back instead of
+// an arrival, a generation and then the read (each a trip of its own, behind a
+// fence of every thread: a Gram-Schmidt sum took 5.5 us of an otherwise empty
+// step on 152 blocks).  A 64-bit value is two 64-bit words of a tag and 32 bits
+// each, so that a word is its own ready flag.  A launch's tags start from the
+// epoch the last one left (one tag per fold); two phases of slots take turns, so
+// a block may run one fold ahead.  Bounded: a wait that gives up sets
+// kStatusSpinTimeout, and every block leaves at its next fold.
+constexpr int kFoldCap = 2 * kLdT;  // values of one fold at most
+struct FoldSlots {
+  unsigned *epoch;
+  ulonglong2 *slot;  // two phases of kFoldCap x gridDim.x, two of kFoldCap sums, kLdT single values
+};
+inline size_t fold_bytes(int blocks) { return 16 + sizeof(ulonglong2) * (2 * (size_t)kFoldCap * (blocks + 1) + kLdT); }
+static inline FoldSlots fold_slots(void *buf) { return FoldSlots{(unsigned *)buf, (ulonglong2 *)((char *)buf + 16)}; }
+
+__device__ __forceinline__ void tag_put(ulonglong2 *p, double v, unsigned tag) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v), t = (unsigned long long)tag << 32;
+  asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(t | (b & 0xffffffffull)), "l"(t | (b >> 32))
+               : "memory");
+}
+__device__ __forceinline__ ulonglong2 tag_load(const ulonglong2 *p) {
+  ulonglong2 v;
+  asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ bool tag_is(ulonglong2 v, unsigned tag) {
+  return (unsigned)(v.x >> 32) == tag && (unsigned)(v.y >> 32) == tag;
+}
+__device__ __forceinline__ double tag_value(ulonglong2 v) {
+  return __longlong_as_double((long long)((v.x & 0xffffffffull) | (v.y << 32)));
+}
+__device__ __forceinline__ bool tag_gave_up(int spins, Control *ctrl) {
+  if (spins <= kMaxSpins && !((spins & 1023) == 1023 && (ld_relaxed(&ctrl->status) & kStatusSpinTimeout))) return false;
+  atomicOr(&ctrl->status, kStatusSpinTimeout);
+  return true;
+}
+// one tagged value, waited for
+__device__ __forceinline__ double tag_get(const ulonglong2 *p, unsigned tag, Control *ctrl, bool &ok) {
+  ulonglong2 v = tag_load(p);
+  for (int spins = 0; !tag_is(v, tag); ++spins) {
+    if (tag_gave_up(spins, ctrl)) {
+      ok = false;
+      break;
+    }
+    v = tag_load(p);
+  }
+  return tag_value(v);
+}
+// the lane's part of a sum over the blocks: p[b] for b = lane, lane + 32, ...
+// added in that order
+__device__ __forceinline__ double tag_lane_sum(const ulonglong2 *p, int blocks, unsigned tag, Control *ctrl, bool &ok) {
+  double t = 0.0;
+  for (int b0 = threadIdx.x & 31; b0 < blocks; b0 += 160) {
+    ulonglong2 v[5];
+    for (int spins = 0;; ++spins) {
+      bool wait = false;
+#pragma unroll
+      for (int u = 0; u < 5; ++u)
+        if (b0 + 32 * u < blocks) v[u] = tag_load(p + b0 + 32 * u);
+#pragma unroll
+      for (int u = 0; u < 5; ++u)
+        if (b0 + 32 * u < blocks) wait |= !tag_is(v[u], tag);
+      if (!wait) break;
+      if (tag_gave_up(spins, ctrl)) {
+        ok = false;
+        break;
       }
     }
-    s_ok = ok;
+#pragma unroll
+    for (int u = 0; u < 5; ++u)
+      if (b0 + 32 * u < blocks) t += tag_value(v[u]);
+  }
+  return t;
+}
+
+// ------------------------------------- shared by the one-kernel steps
+
+// sum_k V[k][i] c[k] over k < ncols: eight independent loads in flight
+__device__ __forceinline__ double vcomb8(const double *__restrict__ V, size_t ldv, int i, int ncols,
+                                         const double *c) {
+  double a[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  int k = 0;
+  for (; k + 8 <= ncols; k += 8) {
+#pragma unroll
+    for (int u = 0; u < 8; ++u) a[u] = fma(V[(size_t)(k + u) * ldv + i], c[k + u], a[u]);
+  }
+#pragma unroll
+  for (int u = 0; u < 8; ++u)
+    if (k + u < ncols) a[u] = fma(V[(size_t)(k + u) * ldv + i], c[k + u], a[u]);
+  return ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
+}
+
+// rows i, i+1 (i even, i+1 < n): sum_k V[k][i..i+1] c[k] over k < ncols with
+// 16-byte loads, a batch of eight columns in flight before any use
+__device__ __forceinline__ double2 vcomb8x2(const double *__restrict__ V, size_t ldv, int i, int ncols,
+                                           const double *c) {
+  // two accumulators per row: the FP64 unit is the scarce one, so few
+  // closing additions matter more than a short dependency chain
+  double2 a[2] = {{0.0, 0.0}, {0.0, 0.0}};
+  for (int k = 0; k < ncols; k += 8) {
+    // a partial batch skips its missing columns
+    double2 v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (k + u < ncols) v[u] = __ldg(reinterpret_cast<const double2 *>(V + (size_t)(k + u) * ldv + i));
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (k + u < ncols) {
+        a[u & 1].x = fma(v[u].x, c[k + u], a[u & 1].x);
+        a[u & 1].y = fma(v[u].y, c[k + u], a[u & 1].y);
+      }
+  }
+  return make_double2(a[0].x + a[1].x, a[0].y + a[1].y);
+}
+
+// block partial sums sacc[k] = sum over this block's rows i > lo of
+// V[k][i] w[i], k < jp1: up to 32 columns as (column, row group) pairs over
+// the 32 warps, more as up to five columns per warp; lanes walk rows
+__device__ __forceinline__ void hh_block_dots(const double *__restrict__ V, size_t ldv, int jp1, int r0, int r1,
+                                              int lo, const double *sw, double *swarp, double *sacc) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int nsl = r1 > r0 ? (r1 - r0 + 31) >> 5 : 0;
+  if (jp1 <= 32) {
+    // row groups per column: no more than have eight slices each to load at once
+    // (every group costs a warp's FP64 sum and an addition)
+    const int G = max(1, min(32 / jp1, nsl >> 3));
+    double acc = 0.0;
+    if (wid < G * jp1) {
+      // a warp streams its column over 1/G of the rows: eight rows per lane
+      // in flight (one block per SM has few warps to hide the latency)
+      const int k = wid % jp1, g = wid / jp1;
+      const double *Vk = V + (size_t)k * ldv + r0;
+      for (int sl0 = g; sl0 < nsl; sl0 += 8 * G) {
+        double v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const int t = 32 * (sl0 + u * G) + lane;
+          v[u] = (sl0 + u * G < nsl && r0 + t < r1) ? Vk[t] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const int t = 32 * (sl0 + u * G) + lane;
+          const int i = r0 + t;
+          acc = fma(v[u], (sl0 + u * G < nsl && i < r1 && i > lo) ? sw[t] : 0.0, acc);
+        }
+      }
+      acc = warp_sum(acc);
+    }
+    if (lane == 0) swarp[wid] = acc;
+    __syncthreads();
+    if (threadIdx.x < jp1) {
+      double t = 0.0;
+      for (int g = 0; g < G; ++g) t += swarp[g * jp1 + threadIdx.x];
+      sacc[threadIdx.x] = t;
+    }
+  } else {
+    double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    for (int sl0 = 0; sl0 < nsl; sl0 += 4) {
+      // four rows per lane for each of the warp's columns in flight
+      double wv[4];
+      int ii[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int t = 32 * (sl0 + u) + lane;
+        const int i = r0 + t;
+        const bool ok = sl0 + u < nsl && i < r1 && i > lo;
+        wv[u] = ok ? sw[t] : 0.0;
+        ii[u] = ok ? i : r0;
+      }
+#pragma unroll
+      for (int c = 0; c < 5; ++c) {
+        const int k = wid + 32 * c;
+        if (32 * c < jp1 && k < jp1) {
+          double v[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) v[u] = V[(size_t)k * ldv + ii[u]];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) acc[c] = fma(v[u], wv[u], acc[c]);
+        }
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 5; ++c) {
+      const int k = wid + 32 * c;
+      if (32 * c < jp1) {  // warp-uniform
+        const double v = warp_sum(acc[c]);
+        if (lane == 0 && k < jp1) swarp[k] = v;
+      }
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < jp1; k += blockDim.x) sacc[k] = swarp[k];
   }
   __syncthreads();
-  return s_ok != 0;
+}
+
+// sres[k] = sum over the grid of the blocks' sacc[k], k < nv, the same in
+// every block.  One or two values: every block adds all partial sums (a warp
+// per value).  More: block k adds value k's and hands the sum out, two trips
+// through L2 - every block adding every value costs ten FP64 instructions of a
+// warp per value and block, 16 cycles of the SM's FP64 unit each (at 31 values
+// 5 us more).  ntop > 0: the rows top0..top1-1 of w that this block owns go out
+// as well, and sres gets rows 0..ntop-1 from position nv on.
+__device__ __forceinline__ bool hh_grid_fold(const double *sacc, int nv, const FoldSlots &f, unsigned tag, Control *ctrl,
+                                             double *sres, const double *stop = nullptr, int top0 = 0, int top1 = 0,
+                                             int ntop = 0) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int G = gridDim.x;
+  ulonglong2 *P = f.slot + (size_t)(tag & 1) * kFoldCap * G;
+  ulonglong2 *R = f.slot + (2 * (size_t)G + (tag & 1)) * kFoldCap, *top = f.slot + (2 * (size_t)G + 2) * kFoldCap;
+  for (int k = top0 + (int)threadIdx.x; k < top1; k += blockDim.x) tag_put(top + k, stop[k - top0], tag);
+  for (int k = threadIdx.x; k < nv; k += blockDim.x) tag_put(P + (size_t)k * G + blockIdx.x, sacc[k], tag);
+  bool ok = true;
+  const bool all = nv <= 2;
+  for (int k = all ? wid : (int)blockIdx.x + wid * G; k < nv; k += (int)(blockDim.x >> 5) * (all ? 1 : G)) {
+    const double t = warp_sum(tag_lane_sum(P + (size_t)k * G, G, tag, ctrl, ok));
+    if (lane == 0) {
+      if (all) sres[k] = t;
+      else tag_put(R + k, t, tag);
+    }
+  }
+  if (!all)
+    for (int k = threadIdx.x; k < nv; k += blockDim.x) sres[k] = tag_get(R + k, tag, ctrl, ok);
+  for (int k = threadIdx.x; k < ntop; k += blockDim.x) sres[nv + k] = tag_get(top + k, tag, ctrl, ok);
+  return __syncthreads_and(ok);
 }
 
 // ------------------------------------------------------------ host side
@@ -257,5 +453,10 @@ static inline int wave_grid(K kernel, int cap) {
   }
   return std::max(1, std::min(cap, per_sm * num_sms()));
 }
+
+// Rows of w (or u) per block of a one-kernel step, a multiple of 32: as many
+// blocks as SMs, but at least 256 rows each - more blocks on a small system only
+// make every sum over them longer.
+static inline int step_rows(int n, int sms) { return std::max(256, ((n + sms - 1) / sms + 31) / 32 * 32); }
 
 }  // namespace lace
