@@ -281,15 +281,19 @@ __global__ void __launch_bounds__(32 * (kGW + kGHelpers)) k_sptrsv_grid(GridArgs
   }
   bool waited = !A.early;
   while (true) {
-    if (rank == 0 && threadIdx.x == 0) {
-      const int t = ngroups > 1 ? atomicAdd(&A.tickets[0], 1) : 0;
-      cl.sync();  // every CTA of the cluster is done with its last tiles, its faces are unsolved
-      for (int r = 0; r < csize; ++r) *(volatile int *)cl.map_shared_rank(&s_tile, r) = t;
-    } else {
-      cl.sync();
+    int tk = 0;
+    if (ngroups > 1) {
+      if (rank == 0 && threadIdx.x == 0) tk = atomicAdd(&A.tickets[0], 1);
+      __syncwarp();
+      tk = __shfl_sync(0xffffffffu, tk, 0);
     }
-    cl.sync();
-    const int tk = *(const volatile int *)&s_tile;
+    cl.sync();  // every CTA of the cluster is done with its last tiles, its faces are unsolved
+    if (ngroups > 1) {
+      if (rank == 0 && (int)threadIdx.x < csize) *(volatile int *)cl.map_shared_rank(&s_tile, threadIdx.x) = tk;
+      __syncwarp();
+      cl.sync();
+      tk = *(const volatile int *)&s_tile;
+    }
     if (tk >= ngroups) break;  // the same for the whole cluster
     const int gy = g.sy / g.cy;
     const int sy_ = tk % gy * g.cy + ry_, sz_ = tk / gy * g.cz + rz_;  // this CTA's super-tile
