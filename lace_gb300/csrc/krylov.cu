@@ -417,7 +417,8 @@ __global__ void __launch_bounds__(kTPB, NS <= 4 ? 3 : 1) k_passB(int n, const do
     }
     __syncthreads();
     tile_dots<NS>(V, ldv, jp1, n, base, kTPB, jp1, sw, acc);
-    tile_dots<NS>(V, ldv, jp1, n, base + kTPB, kTPB, jp1, sw + kTPB, acc);
+    // (a half tile past the last row would read the next column's first rows, not written yet)
+    if (base + kTPB < n) tile_dots<NS>(V, ldv, jp1, n, base + kTPB, kTPB, jp1, sw + kTPB, acc);
   }
   block_reduce_slots<NS>(acc, jp1, sred);
   double tot = block_sum(nrm, scratch);
