@@ -425,7 +425,9 @@ int lace_gpu_apply_precond(lace_gpu_ctx *ctx, const double *q, double *z);
  * out[0] rows per lane, out[1] chunks per block, out[2] warps per CTA,
  * out[3] CTAs per thread-block cluster (1: none).  For the factors of a 5- or
  * 7-point grid in natural order, solved a lane per grid line: out[0] the rows
- * of a line, out[1] and out[2] the tiles (warps) per CTA, out[3] as above.
+ * of a line, out[1] and out[2] the tiles (warps) per CTA, out[3] as above.  For
+ * solves whose rows push their values to the rows that wait for them: out[0] 1,
+ * out[1] 0, out[2] warps per CTA, out[3] CTAs (one cluster).
  * DEV_ERR_NOT_INITIALIZED before.  No counterpart in LACE. */
 int lace_gpu_get_trsv_schedule(lace_gpu_ctx *ctx, int *out);
 

@@ -534,6 +534,103 @@ int lace_gpu_ctx::ensure_grid(int which) {
   return cudaGetLastError() == cudaSuccess ? 0 : DEV_ERR_UNKNOWN;
 }
 
+// The solves with pushed values, on the fewest CTAs that hold the slots and on
+// twice as many (more of the pushes are far ones then, but a level's groups have
+// more warps): the faster one's plans, and the time of two pairs.  Where the
+// triangles do not fit push_C is 0.
+int lace_gpu_ctx::try_push(float *ms) {
+  *ms = 1e30f;
+  const Pattern *pats[2] = {&hL, &hU};
+  const size_t ct = vtype() == VType::F64 ? 8 : 4;
+  const int f32 = ct == 4;
+  push_C = 0;
+  for (int w = 0; w < 4; ++w) {
+    pplans[w].valid = false;
+    push_unfit[w] = false;
+  }
+  if (opt.trsv_chunks_per_block > 0 || opt.trsv_rows_per_lane > 0 || opt.trsv_warps > 0 || opt.trsv_cluster > 0) return 0;
+  cudaEvent_t e0, e1;
+  cudaEventCreate(&e0);
+  cudaEventCreate(&e1);
+  int rc = 0, tried = 0, best = 0, last = 0;
+  for (int C = 1; C <= 16 && tried < 2 && !rc; C *= 2) {
+    PushHost h[2];
+    int no[2] = {0, 0};
+    std::thread other([&] { no[1] = push_plan_host(*pats[1], false, std::max(bs, 1), ct, C, h[1]); });
+    no[0] = push_plan_host(*pats[0], true, std::max(bs, 1), ct, C, h[0]);
+    other.join();
+    if (std::max(no[0], no[1]) == 2) break;
+    if (no[0] || no[1]) continue;
+    ++tried;
+    for (int w = 0; w < 2 && !rc; ++w) rc = push_plan_upload(stream, h[w], std::max(bs, 1), ct, C, w == 0, pplans[w]);
+    if (rc || !pplans[0].valid || !pplans[1].valid) continue;
+    push_C = last = C;
+    for (int r = 0; r < 3 && !rc; ++r) {
+      if (r == 1) cudaEventRecord(e0, stream);
+      rc = solve_pair(0, 1, vec_q.p, f32, vec_r.p, f32, false, false);
+    }
+    cudaEventRecord(e1, stream);
+    if (cudaEventSynchronize(e1) != cudaSuccess) rc = DEV_ERR_UNKNOWN;
+    float t = 1e30f;
+    if (!rc) cudaEventElapsedTime(&t, e0, e1);
+    if (h_status() & kStatusSpinTimeout) {
+      cudaMemsetAsync(&ctrl()->status, 0, 4, stream);
+      t = 1e30f;
+    }
+    if (verbose) printf("trsv autotune pushed values on %d CTAs, %d levels: %.3f ms per pair\n", C, h[0].levels, t / 2);
+    if (t < *ms) {
+      *ms = t;
+      best = C;
+    }
+  }
+  cudaEventDestroy(e0);
+  cudaEventDestroy(e1);
+  push_C = best;
+  if (best != last)
+    for (auto &p : pplans) p.valid = false;  // built again for the chosen size
+  return rc || !best ? rc : ready_tri(0, 1);
+}
+
+// the plans of two triangles with the current values, ahead of a capture
+int lace_gpu_ctx::ready_tri(int t1, int t2) {
+  if (opt.trsv_mode != LACE_TRSV_SYNCFREE) return 0;
+  for (int t : {t1, t2}) {
+    bool on = false;
+    int rc = ensure_push(t, &on);
+    if (!rc && !on && !bs) rc = ensure_plan(t);
+    if (rc) return rc;
+  }
+  return 0;
+}
+
+// triangle which's plan on push_C CTAs with the current values; *on: it has one
+int lace_gpu_ctx::ensure_push(int which, bool *on) {
+  *on = false;
+  if (!push_C || opt.trsv_mode != LACE_TRSV_SYNCFREE || push_unfit[which]) return 0;
+  PushPlan &p = pplans[which];
+  const TriDev t = tri(which);
+  if (!p.valid) {
+    const Pattern *pats[4] = {&hL, &hU, &hUc, &hLt};
+    const size_t ct = vtype() == VType::F64 ? 8 : 4;
+    PushHost h;
+    if (!push_plan_host(*pats[which], t.lower != 0, std::max(bs, 1), ct, push_C, h)) {
+      const int rc = push_plan_upload(stream, h, std::max(bs, 1), ct, push_C, t.unit != 0, p);
+      if (rc) return rc;
+    }
+    if (!p.valid) {
+      push_unfit[which] = true;
+      return 0;
+    }
+  }
+  if (p.vals_version != fact_version || p.vals_src != t.val) {
+    launch_push_values(stream, p, t.val, dinv.p, vtype());
+    p.vals_version = fact_version;
+    p.vals_src = t.val;
+  }
+  *on = true;
+  return cudaGetLastError() == cudaSuccess ? 0 : DEV_ERR_UNKNOWN;
+}
+
 int lace_gpu_ctx::limit_reached() {
   for (auto &p : gplans)
     if (p.valid) grid_clear_faces(stream, p);
@@ -544,6 +641,16 @@ int lace_gpu_ctx::solve_pair(int t1, int t2, const void *b, int in_f32, void *z,
                              bool prefilled) {
   const int f32 = vtype() != VType::F64;  // the vector between the triangles
   if (!(grid_on && syncfree_blocks())) {
+    bool on1 = false, on2 = false;
+    int rp = ensure_push(t1, &on1);
+    if (!rp && on1) rp = ensure_push(t2, &on2);
+    if (rp) return rp;
+    if (on1 && on2) {
+      Control *cb = ctrl();
+      const int *done = honor_done ? &cb->done : nullptr;
+      rp = launch_push(stream, pplans[t1], b, in_f32, vec_t.p, f32, 0, &cb->status, done);
+      return rp ? rp : launch_push(stream, pplans[t2], vec_t.p, f32, z, z_f32, 1, &cb->status, done);
+    }
     const int rc = solve_tri(t1, b, in_f32, vec_t.p, f32, honor_done, vec_t2.p, prefilled);
     return rc ? rc : solve_tri(t2, vec_t.p, f32, z, z_f32, honor_done, vec_t2.p, prefilled);
   }
@@ -919,6 +1026,7 @@ int lace_gpu_ctx::analyse_factors(const Pattern &L, const Pattern &Ur) {
   factors_ready = false;
   trsv_tuned = false;
   bcsr_tuned = false;
+  push_C = 0;
   ws_m = 0;
   drop_graphs();
   return 0;
@@ -1567,6 +1675,11 @@ int lace_gpu_ctx::solve_tri(int which, const void *b, int in_f32, void *x, int o
       launch_convert(stream, n, in_f32 ? VType::F32 : VType::F64, b, out_f32 ? VType::F32 : VType::F64, x);
       break;
     default:
+      bool pushed = false;
+      if (const int rc = ensure_push(which, &pushed)) return rc;
+      if (pushed)
+        return launch_push(stream, pplans[which], b, in_f32, x, out_f32, 0, &cb->status,
+                           honor_done ? &cb->done : nullptr);
       if (bs) {
         if (b == x) {  // the solve fills x before it reads b
           cudaMemcpyAsync(tmp, b, (size_t)n * (in_f32 ? 4 : 8), cudaMemcpyDeviceToDevice, stream);
@@ -1613,12 +1726,17 @@ int lace_gpu_ctx::autotune_bcsr_trsv() {
   if (rc) return rc;
   const int f32 = vtype() != VType::F64;
   cudaMemsetAsync(vec_q.p, 0, 8 * (size_t)n, stream);
+  float push_ms = 1e30f;
+  if ((rc = try_push(&push_ms))) return rc;
+  const int pushed = push_C;
+  push_C = 0;
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
   float best = 1e30f;
   int best_grid = num_sms() * 8;
-  for (int per_sm : {2, 4, 8}) {
+  for (int per_sm : {4, 2, 8}) {
+    if (best > 1.5f * push_ms && best < 1e30f) break;  // the three lie within a few percent of one another
     bcsr_grid = num_sms() * per_sm;
     float ms = 0.f;
     for (int rep = 0; rep < 3 && !rc; ++rep) {
@@ -1643,7 +1761,9 @@ int lace_gpu_ctx::autotune_bcsr_trsv() {
   bcsr_grid = best_grid;
   if (rc) return rc;
   if (h_status() & kStatusSpinTimeout) return DEV_ERR_INTERNAL_LIMIT;
+  if (push_ms < best) push_C = pushed;
   bcsr_tuned = true;
+  drop_graphs();
   return 0;
 }
 
@@ -1652,6 +1772,7 @@ int lace_gpu_ctx::autotune_trsv() {
   if (bs || opt.trsv_mode != LACE_TRSV_SYNCFREE) return 0;
   if (trsv_tuned) return 0;
   int rc = ensure_vectors();
+  push_C = 0;
   if (!rc) rc = try_grid();
   if (rc) return rc;
   if (grid_on) {
@@ -1661,10 +1782,14 @@ int lace_gpu_ctx::autotune_trsv() {
   }
   const bool f32 = vtype() != VType::F64;
   cudaMemsetAsync(vec_q.p, 0, 8 * (size_t)n, stream);
+  float best = 1e30f;
+  if ((rc = try_push(&best))) return rc;
+  const int pushed = push_C;
+  push_C = 0;
+  const float push_ms = best;
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
-  float best = 1e30f;
   int bR = 4, bC = 1, bW = 1, bL = 1;
   // schedule shapes: (rows per lane, chunks per block, warps per CTA, CTAs
   // per cluster); a block of one chunk on one warp is the warp-level
@@ -1702,8 +1827,9 @@ int lace_gpu_ctx::autotune_trsv() {
   // times stay within about 15 % of one another, are built and timed only if
   // the representative comes within 1.5x of the best so far.
   auto family = [](const Cand &c) { return c.cpb == 1 ? 3 : (c.R == 1 ? 0 : (c.R == 2 ? 1 : 2)); };
-  const Cand reps[4] = {{1, 0, 0, 0}, {2, 256, 16, 1}, {4, 128, 16, 1}, {1, 1, 1, 1}};
-  for (int f = 1; f < 4; ++f) {
+  const Cand reps[4] = {{1, 256, 16, 1}, {2, 256, 16, 1}, {4, 128, 16, 1}, {1, 1, 1, 1}};
+  // (with pushed values in the lead the first family, too)
+  for (int f = pushed ? 0 : 1; f < 4; ++f) {
     bool have_rep = false;
     for (auto &c : cands)
       have_rep |= family(c) == f && c.R == reps[f].R && c.cpb == reps[f].cpb && c.w == reps[f].w && c.cl == reps[f].cl;
@@ -1714,7 +1840,7 @@ int lace_gpu_ctx::autotune_trsv() {
                                         c.cl == reps[f].cl)
                                      : first;
         first = false;
-        c.grp = is_rep ? 2 * f - 1 : 2 * f;
+        c.grp = is_rep ? 2 * (f + 1) - 1 : 2 * (f + 1);
       }
   }
   for (auto &c : cands) c.fam = family(c);
@@ -1833,6 +1959,7 @@ int lace_gpu_ctx::autotune_trsv() {
   trsv_tuned = true;
   cudaMemsetAsync(&ctrl()->status, 0, 4, stream);
   drop_graphs();
+  if (pushed && best >= push_ms) push_C = pushed;
   if (best >= 1e30f) return DEV_ERR_INTERNAL_LIMIT;  // no shape finished its solves
   return cudaGetLastError() == cudaSuccess ? 0 : DEV_ERR_UNKNOWN;
 }
@@ -1877,6 +2004,13 @@ extern "C" int lace_gpu_get_trsv_schedule(lace_gpu_ctx *c, int *out) {
     out[0] = c->grid.nx;
     out[1] = out[2] = c->grid.wy * c->grid.wz;
     out[3] = c->grid.cy * c->grid.cz;
+    return DEV_SUCCESS;
+  }
+  if (c->push_C) {  // a lane per row, no blocks
+    out[0] = 1;
+    out[1] = 0;
+    out[2] = lace::kPushW;
+    out[3] = c->push_C;
     return DEV_SUCCESS;
   }
   out[0] = c->plan_R;
@@ -2052,7 +2186,7 @@ ArnoldiArgs lace_gpu_ctx::arnoldi_args(int m, bool adjoint) {
   a.cy = (Cycle *)cycle_buf.p;
   a.ctrl = ctrl();
   a.m = m;
-  a.prefill = syncfree_blocks() && !grid_on ? 1 : 0;
+  a.prefill = syncfree_blocks() && !grid_on && !push_C ? 1 : 0;
   a.fill_t = vec_t.p;
   a.fill_t_f32 = vtype() != VType::F64 ? 1 : 0;
   return a;
@@ -2186,10 +2320,7 @@ int lace_gpu_ctx::fgmres(const double *b, double *x, int m, int restart_max, int
   if (!rc && !adjoint) rc = ensure_sell();
   sc.mark("operator (A^T or sliced ELL)");
   // solve plans are built on the host: before any graph capture
-  if (!rc && !bs && opt.trsv_mode == LACE_TRSV_SYNCFREE) {
-    rc = ensure_plan(adjoint ? 2 : 0);
-    if (!rc) rc = ensure_plan(adjoint ? 3 : 1);
-  }
+  if (!rc) rc = ready_tri(adjoint ? 2 : 0, adjoint ? 3 : 1);
   if (!rc && cudaStreamSynchronize(stream) != cudaSuccess) rc = DEV_ERR_UNKNOWN;
   if (rc) return rc;
   sc.mark("solve plans");

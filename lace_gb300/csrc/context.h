@@ -63,6 +63,30 @@ int launch_grid_pair(cudaStream_t s, GridPlan &p1, GridPlan &p2, const void *b, 
 int launch_grid_tri(cudaStream_t s, GridPlan &p, const void *b, int in_f32, void *t, void *x, int out_f32, int *status,
                     const int *done);
 
+// one triangle's plan with pushed values on C CTAs (sptrsv_push.cu), per group
+// of 32 / bs rows; dst: CTA << 24 | byte offset of the slot of component 0
+constexpr int kPushW = 16;  // warps per CTA
+struct PushHost {
+  int K = 0, groups = 0, levels = 0;
+  size_t smem = 0;
+  std::vector<int> wptr, slot, rc, dst, map, dmap;
+};
+struct PushPlan {
+  bool valid = false;
+  int bs = 1, C = 1, K = 4, groups = 0, unit = 0;
+  size_t smem = 0, ct = 4;
+  DBuf wptr, slot, rc, dst, map, dmap, val, rd;
+  int vals_version = -1;
+  const void *vals_src = nullptr;
+};
+int push_plan_host(const Pattern &T, bool lower, int bs, size_t ct, int C, PushHost &h);
+// leaves the plan invalid where the device has no room for its cluster
+int push_plan_upload(cudaStream_t s, const PushHost &h, int bs, size_t ct, int C, bool unit, PushPlan &p);
+void launch_push_values(cudaStream_t s, PushPlan &p, const void *val, const void *dinv, VType vt);
+// early: the kernel before is the pair's first triangle
+int launch_push(cudaStream_t s, const PushPlan &p, const void *b, int in_f32, void *x, int out_f32, int early,
+                int *status, const int *done);
+
 // host part of a plan (what build_blk_plan_host fills, upload_blk_plan sends)
 struct HostPlan {
   int n = 0, nch = 0, R = 1, cpb = 1, max_units = 0;
@@ -152,6 +176,13 @@ struct lace_gpu_ctx {
   lace::GridPlan gplans[4];
   lace::DBuf grid_t;  // the vector between the two triangles, in tile order
   int try_grid();
+  // the solves with pushed values (sptrsv_push.cu), chosen by time; CTAs a triangle (0: none)
+  int push_C = 0;
+  lace::PushPlan pplans[4];
+  bool push_unfit[4] = {false, false, false, false};
+  int try_push(float *ms);
+  int ensure_push(int which, bool *on);
+  int ready_tri(int t1, int t2);
   int ensure_grid(int which);
   int limit_reached();  // DEV_ERR_INTERNAL_LIMIT, after making the grid plans usable again
   // z = T2^{-1} T1^{-1} b for two consecutive triangles (L and U, or U^T and L^T)
