@@ -6,12 +6,17 @@
 // the A-order ParILU records for all of them at once) and, per system, the
 // level sets of its two triangles.  lace_gpu_batch_solve then runs the whole
 // solve - every system's ParILU sweeps and FGMRES-Householder for every
-// (system, rhs) pair - as one persistent launch (batch_persist.cu), captured
-// in a CUDA graph when the context's options ask for graphs.
+// (system, rhs) pair - as one persistent launch, captured in a CUDA graph when
+// the context's options ask for graphs: a cluster of CTAs per pair
+// (batch_cluster.cu), or, where a system's triangles do not fit a cluster's
+// shared memory, a CTA per system and up to four of its right-hand sides
+// (batch_persist.cu).
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <atomic>
 #include <numeric>
+#include <thread>
 #include <vector>
 
 #include "context.h"
@@ -32,6 +37,12 @@ struct lace_gpu_batch {
   DBuf F;                                                // per CTA: factor values in A's order, twice
   DBuf V, W, Tm, Rm, Z, Q, Tt, ctl;                              // per-CTA workspace, queue and results
   int grid = 0, m = 0, f32 = -1;
+  // the cluster form: the block-diagonal pattern, and per triangle (0 L, 1 U)
+  // the systems' plans one after the other
+  std::vector<int> hrow, hcol;
+  int C = 0, K = 2, plan_ct = 0, clusters = 0, gmax[2] = {0, 0}, rbmax = 0;
+  size_t slot_bytes = 0, csmem = 0;
+  DBuf wptr[2], goff[2], pslot[2], rc[2], dst[2], map[2], dmap[2], cjsys, cjrhs, vals;
 };
 
 namespace {
@@ -211,8 +222,175 @@ extern "C" int lace_gpu_batch_create(lace_gpu_batch **out, lace_gpu_ctx *ctx, in
     delete B;
     return set_err(DEV_ERR_UNKNOWN);
   }
+  B->hrow = std::move(Sr);
+  B->hcol = std::move(Sc);
   *out = B;
   return DEV_SUCCESS;
+}
+
+// CTAs per cluster (1, 2, 4, 8) by the time the queue takes: per search
+// direction a job costs 26 ns a row divided over the CTAs (the FP64 units'
+// share at 15 basis vectors), 0.18 us a level of its triangles and 10 us of
+// barriers and small matrices (all measured), and a grid's directions grow with
+// its side; the clusters side by side take the jobs' sum, and none less than
+// the largest job.  24 systems of up to 9,025 rows, four right-hand sides: C = 1,
+// 2, 4, 8 at 93, 45, 37 and 75 ms.
+static double cluster_cost(const lace_gpu_batch *B, const std::vector<int> &levels, int C) {
+  double sum = 0.0, top = 0.0;
+  for (int s = 0; s < B->nsys; ++s) {
+    const double t = std::sqrt((double)B->n[s]) * (0.026 * B->n[s] / C + 0.18 * levels[s] + 10.0);
+    sum += t * B->nrhs;
+    top = std::max(top, t);
+  }
+  return std::max(top, sum / std::max(1, num_sms() / C));
+}
+
+// The cluster form's plans for value size ct and m directions (C = 0: the
+// batch does not fit it).
+static int cluster_plan(lace_gpu_batch *B, int m, size_t ct) {
+  if (B->plan_ct == (int)ct && B->m == m) return 0;
+  B->C = 0;
+  B->plan_ct = 0;
+  lace_gpu_ctx *c = B->ctx;
+  const int nsys = B->nsys;
+  // the triangles of each system and their entries' positions in A
+  struct Sys {
+    Pattern T[2];
+    std::vector<int> pos[2];
+    PushHost h[2];
+    int levels = 0, fit = 0;
+  };
+  std::vector<Sys> S(nsys);
+  auto parallel = [&](auto fn) {
+    std::atomic<int> next{0};
+    auto work = [&] {
+      for (int s; (s = next.fetch_add(1)) < nsys;) fn(s);
+    };
+    std::vector<std::thread> th;
+    const int k = std::min(nsys, std::max(1, std::min(16, (int)std::thread::hardware_concurrency())));
+    for (int i = 1; i < k; ++i) th.emplace_back(work);
+    work();
+    for (auto &x : th) x.join();
+  };
+  parallel([&](int s) {
+    const int n = B->n[s], r0 = B->row_off[s];
+    for (int up = 0; up < 2; ++up) {
+      Pattern &T = S[s].T[up];
+      T.n = n;
+      T.ptr.assign(1, 0);
+      for (int i = 0; i < n; ++i) {
+        for (int p = B->hrow[r0 + i]; p < B->hrow[r0 + i + 1]; ++p) {
+          const int j = B->hcol[p] - r0;
+          if (up ? j < i : j > i) continue;
+          T.idx.push_back(j);
+          S[s].pos[up].push_back(p);
+        }
+        T.ptr.push_back((int)T.idx.size());
+      }
+      std::vector<int> lev(n, 0);
+      int d = 0;
+      for (int k = 0; k < n; ++k) {
+        const int i = up ? n - 1 - k : k;
+        for (int e = T.ptr[i]; e < T.ptr[i + 1]; ++e)
+          if (T.idx[e] != i) lev[i] = std::max(lev[i], lev[T.idx[e]] + 1);
+        d = std::max(d, lev[i] + 1);
+      }
+      S[s].levels += d;
+    }
+  });
+  std::vector<int> levels(nsys);
+  for (int s = 0; s < nsys; ++s) levels[s] = S[s].levels;
+  std::vector<int> order{1, 2, 4, 8};
+  std::stable_sort(order.begin(), order.end(),
+                   [&](int a, int b) { return cluster_cost(B, levels, a) < cluster_cost(B, levels, b); });
+  for (int C : order) {
+    int rb = 0;
+    const size_t rest = batch_cluster_smem(0, B->nmax, m, C, &rb);
+    if (rest + 1024 > batch_cluster_smem_max()) continue;
+    const size_t cap = batch_cluster_smem_max() - rest;
+    int K = 2;
+    for (bool again = true; again;) {
+      again = false;
+      parallel([&](int s) {
+        // the fewest CTAs that hold the slots of both triangles
+        Sys &y = S[s];
+        y.fit = 0;
+        for (int ctas = 1; ctas <= C && !y.fit; ctas *= 2) {
+          int no = 0;
+          for (int up = 0; up < 2 && !no; ++up) {
+            y.h[up] = PushHost();
+            y.h[up].K = K;
+            no = push_plan_host(y.T[up], up == 0, 1, ct, ctas, y.h[up]);
+            if (!no && y.h[up].smem > cap) no = 1;
+          }
+          if (!no) y.fit = ctas;
+          if (no == 2) break;
+        }
+      });
+      int kmax = K;
+      for (auto &y : S)
+        if (y.fit) kmax = std::max({kmax, y.h[0].K, y.h[1].K});
+      if (kmax > 4) return 0;
+      if (kmax > K) {
+        K = 4;
+        again = true;
+      }
+    }
+    bool fit = true;
+    for (auto &y : S) fit = fit && y.fit;
+    if (!fit) continue;
+    B->slot_bytes = 256;
+    for (int up = 0; up < 2; ++up) {
+      std::vector<int> wptr, goff, slot, rc, dst, map, dmap;
+      B->gmax[up] = 0;
+      for (int s = 0; s < nsys; ++s) {
+        const PushHost &h = S[s].h[up];
+        goff.push_back((int)slot.size());
+        B->gmax[up] = std::max(B->gmax[up], h.groups);
+        B->slot_bytes = std::max(B->slot_bytes, h.smem);
+        wptr.insert(wptr.end(), h.wptr.begin(), h.wptr.end());
+        wptr.resize((size_t)(s + 1) * (C * kPushW + 1), h.groups);  // CTAs without groups
+        slot.insert(slot.end(), h.slot.begin(), h.slot.end());
+        rc.insert(rc.end(), h.rc.begin(), h.rc.end());
+        dst.insert(dst.end(), h.dst.begin(), h.dst.end());
+        for (int e : h.map) map.push_back(e < 0 ? -1 : S[s].pos[up][e]);
+        for (int e : h.dmap) dmap.push_back(e < 0 ? -1 : S[s].pos[up][e]);
+      }
+      auto send = [&](DBuf &d, const std::vector<int> &v) { return d.upload(v.data(), 4 * v.size(), c->stream); };
+      if (send(B->wptr[up], wptr) || send(B->goff[up], goff) || send(B->pslot[up], slot) || send(B->rc[up], rc) ||
+          send(B->dst[up], dst) || send(B->map[up], map) || send(B->dmap[up], dmap) ||
+          cudaStreamSynchronize(c->stream) != cudaSuccess)
+        return DEV_ERR_DEVICE_ALLOC;
+    }
+    // jobs, largest systems first
+    std::vector<int> by(nsys), js, jr;
+    std::iota(by.begin(), by.end(), 0);
+    std::stable_sort(by.begin(), by.end(), [&](int a, int b) { return B->n[a] > B->n[b]; });
+    for (int s : by)
+      for (int r = 0; r < B->nrhs; ++r) {
+        js.push_back(s);
+        jr.push_back(r);
+      }
+    if (B->cjsys.upload(js.data(), 4 * js.size(), c->stream) || B->cjrhs.upload(jr.data(), 4 * jr.size(), c->stream) ||
+        cudaStreamSynchronize(c->stream) != cudaSuccess)
+      return DEV_ERR_DEVICE_ALLOC;
+    B->csmem = batch_cluster_smem(B->slot_bytes, B->nmax, m, C, &B->rbmax);
+    B->K = K;
+    CBatch P = {};
+    P.C = C;
+    P.K = K;
+    P.f32 = ct == 4;
+    P.smem = B->csmem;
+    int room = 0;
+    const int rc = launch_batch_cluster(c->stream, P, 1, &room);
+    if (rc) return rc;
+    if (room < 1) continue;
+    B->clusters = std::max(1, std::min(nsys * B->nrhs, std::min(room, num_sms() / C)));
+    B->C = C;
+    break;
+  }
+  B->plan_ct = (int)ct;
+  return 0;
 }
 
 extern "C" int lace_gpu_batch_destroy(lace_gpu_batch *B) {
@@ -228,6 +406,27 @@ extern "C" int lace_gpu_batch_destroy(lace_gpu_batch *B) {
 // register budget), at most one per system
 static int batch_workspace(lace_gpu_batch *B, int m, bool f32) {
   if (m == B->m && (int)f32 == B->f32 && B->V.p) return 0;
+  B->V.free();
+  const int prc = cluster_plan(B, m, f32 ? 4 : 8);
+  if (prc) return prc;
+  if (B->C) {
+    const size_t G = (size_t)B->clusters, nmax = (size_t)B->nmax, fb = f32 ? 4 : 8;
+    int rc = 0;
+    rc |= B->F.ensure(fb * G * 2 * (B->nnzmax + 4));
+    rc |= B->vals.ensure(fb * G * 32 * ((size_t)(B->gmax[0] + B->gmax[1]) * B->K + B->gmax[1]));
+    rc |= B->Z.ensure(fb * G * m * nmax);
+    rc |= B->Q.ensure(fb * G * nmax);
+    rc |= B->Tt.ensure(fb * G * nmax);
+    rc |= B->ctl.ensure(4 * (2 + 2 * (size_t)B->nsys * B->nrhs));
+    rc |= B->V.ensure(8 * G * (m + 1) * nmax);
+    if (rc) {
+      B->V.free();
+      return DEV_ERR_DEVICE_ALLOC;
+    }
+    B->m = m;
+    B->f32 = f32;
+    return 0;
+  }
   const int R = batch_persist_rhs();
   B->grid = std::max(1, std::min(B->njobs, num_sms()));
   const size_t G = (size_t)B->grid, nmax = (size_t)B->nmax, ld = (size_t)m + 2;
@@ -242,7 +441,7 @@ static int batch_workspace(lace_gpu_batch *B, int m, bool f32) {
   rc |= B->Z.ensure(fb * G * R * m * nmax);
   rc |= B->Q.ensure(fb * G * R * nmax);
   rc |= B->Tt.ensure(fb * G * R * nmax);
-  rc |= B->ctl.ensure(4 * (1 + 2 * (size_t)B->nsys * B->nrhs));
+  rc |= B->ctl.ensure(4 * (2 + 2 * (size_t)B->nsys * B->nrhs));
   if (rc) return DEV_ERR_DEVICE_ALLOC;
   B->m = m;
   B->f32 = f32;
@@ -265,6 +464,57 @@ extern "C" int lace_gpu_batch_solve(lace_gpu_batch *B, int sweeps, int search_ma
   const size_t pairs = (size_t)B->nsys * B->nrhs;
   int *ctl = (int *)B->ctl.p;
   if (cudaMemsetAsync(ctl, 0, B->ctl.bytes, s) != cudaSuccess) return set_err(DEV_ERR_UNKNOWN);
+  CBatch P = {};
+  if (B->C) {
+    P.nrhs = B->nrhs;
+    P.m = search_max;
+    P.restart_max = restart_max;
+    P.sweeps = sweeps;
+    P.N = B->N;
+    P.njobs = (int)pairs;
+    P.C = B->C;
+    P.K = B->K;
+    P.f32 = f32 ? 1 : 0;
+    P.rtol = rtol;
+    P.jsys = (const int *)B->cjsys.p;
+    P.jrhs = (const int *)B->cjrhs.p;
+    P.n = (const int *)B->dn.p;
+    P.roff = (const int *)B->droff.p;
+    P.Arow = (const int *)c->Arow.p;
+    P.Acol = (const int *)c->Acol.p;
+    P.Aval = (const double *)c->Aval.p;
+    P.pptr = (const int *)c->sw_pptr.p;
+    P.dpos = (const int *)c->sw_dpos.p;
+    P.pairs = (const int2 *)c->sw_pairs.p;
+    for (int up = 0; up < 2; ++up) {
+      P.wptr[up] = (const int *)B->wptr[up].p;
+      P.goff[up] = (const int *)B->goff[up].p;
+      P.slot[up] = (const int *)B->pslot[up].p;
+      P.rc[up] = (const int *)B->rc[up].p;
+      P.dst[up] = (const int *)B->dst[up].p;
+      P.map[up] = (const int *)B->map[up].p;
+      P.dmap[up] = (const int *)B->dmap[up].p;
+      P.gmax[up] = B->gmax[up];
+    }
+    P.vstride = 32 * ((size_t)(B->gmax[0] + B->gmax[1]) * B->K + B->gmax[1]);
+    P.fstride = B->nnzmax + 4;
+    P.nmax = (size_t)B->nmax;
+    P.smem = B->csmem;
+    P.slot_bytes = (unsigned)B->slot_bytes;
+    P.rbmax = B->rbmax;
+    P.V = (double *)B->V.p;
+    P.F = B->F.p;
+    P.val = B->vals.p;
+    P.Z = B->Z.p;
+    P.Q = B->Q.p;
+    P.Tt = B->Tt.p;
+    P.b = b;
+    P.x = x;
+    P.next = ctl;
+    P.iters = ctl + 1;
+    P.conv = ctl + 1 + pairs;
+    P.status = ctl + 1 + 2 * pairs;
+  }
   PBatchHost h;
   h.nsys = B->nsys;
   h.nrhs = B->nrhs;
@@ -321,7 +571,7 @@ extern "C" int lace_gpu_batch_solve(lace_gpu_batch *B, int sweeps, int search_ma
     // the one launch, captured and replayed as a graph
     cudaGraph_t g = nullptr;
     if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) != cudaSuccess) return set_err(DEV_ERR_UNKNOWN);
-    rc = launch_batch_persist(s, h);
+    rc = B->C ? launch_batch_cluster(s, P, B->clusters, nullptr) : launch_batch_persist(s, h);
     const cudaError_t ce = cudaStreamEndCapture(s, &g);
     if (rc || ce != cudaSuccess) return set_err(rc ? rc : DEV_ERR_UNKNOWN);
     const cudaError_t ie = cudaGraphInstantiate(&ge, g, 0);
@@ -332,14 +582,15 @@ extern "C" int lace_gpu_batch_solve(lace_gpu_batch *B, int sweeps, int search_ma
       return set_err(DEV_ERR_UNKNOWN);
     }
   } else {
-    rc = launch_batch_persist(s, h);
+    rc = B->C ? launch_batch_cluster(s, P, B->clusters, nullptr) : launch_batch_persist(s, h);
     if (rc) return set_err(rc);
   }
-  std::vector<int> res(2 * pairs);
+  std::vector<int> res(2 * pairs + 1);
   const bool ok = cudaMemcpyAsync(res.data(), ctl + 1, 4 * res.size(), cudaMemcpyDeviceToHost, s) == cudaSuccess &&
                   cudaStreamSynchronize(s) == cudaSuccess;
   if (ge) cudaGraphExecDestroy(ge);
   if (!ok) return set_err(DEV_ERR_UNKNOWN);
+  if (res[2 * pairs] & kStatusSpinTimeout) return set_err(DEV_ERR_INTERNAL_LIMIT);
   bool all = true;
   for (size_t k = 0; k < pairs; ++k) {
     if (iters_out) iters_out[k] = res[k];

@@ -67,7 +67,7 @@ int launch_grid_tri(cudaStream_t s, GridPlan &p, const void *b, int in_f32, void
 // of 32 / bs rows; dst: CTA << 24 | byte offset of the slot of component 0
 constexpr int kPushW = 16;  // warps per CTA
 struct PushHost {
-  int K = 0, groups = 0, levels = 0;
+  int K = 3, groups = 0, levels = 0;  // K: entries a row has room for, at least
   size_t smem = 0;
   std::vector<int> wptr, slot, rc, dst, map, dmap;
 };

@@ -258,6 +258,33 @@ struct PBatchHost {
   int *next = nullptr, *iters = nullptr, *conv = nullptr;
 };
 int launch_batch_persist(cudaStream_t s, const PBatchHost &h);
+// the batched solve with a cluster of C CTAs per job (batch_cluster.cu); plans
+// of the triangles (0 L, 1 U) of all systems one after the other
+struct CBatch {
+  int nrhs, m, restart_max, sweeps, N, njobs, C, K, f32;
+  double rtol;
+  const int *jsys, *jrhs, *n, *roff;
+  const int *Arow, *Acol;
+  const double *Aval;
+  const int *pptr, *dpos;
+  const int2 *pairs;
+  const int *wptr[2], *goff[2], *slot[2], *rc[2], *dst[2], *map[2], *dmap[2];
+  int gmax[2];                  // the largest system's groups
+  size_t vstride, fstride, nmax;  // per cluster: plan values, factor values (two), rows
+  size_t smem;
+  unsigned slot_bytes;
+  int rbmax;
+  double *V;
+  void *F, *val, *Z, *Q, *Tt;
+  const double *b;
+  double *x;
+  int *next, *iters, *conv, *status;
+};
+// shared memory a CTA needs, and the rows of w it keeps
+size_t batch_cluster_smem(size_t slot_bytes, int nmax, int m, int C, int *rbmax);
+size_t batch_cluster_smem_max();
+// launches, or with room set asks for the clusters the device holds
+int launch_batch_cluster(cudaStream_t s, const CBatch &P, int clusters, int *room);
 int batch_persist_threads();
 int batch_persist_rhs();
 void launch_sell_values(cudaStream_t s, size_t count, const int *map, const double *src, double *dst,

@@ -27,52 +27,13 @@
 #include <cooperative_groups.h>
 
 #include "context.h"
+#include "push.cuh"
 
 namespace lace {
 
 namespace {
 
 constexpr size_t kPushSmemMax = 220 * 1024;
-
-// the unsolved mark: all ones, told by the high word
-__device__ __forceinline__ unsigned head(float v) { return __float_as_uint(v); }
-__device__ __forceinline__ unsigned head(double v) { return (unsigned)__double2hiint(v); }
-
-__device__ __forceinline__ float ld_slot(unsigned a, float) {
-  float v;
-  asm volatile("ld.volatile.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
-  return v;
-}
-__device__ __forceinline__ double ld_slot(unsigned a, double) {
-  double v;
-  asm volatile("ld.volatile.shared.f64 %0, [%1];" : "=d"(v) : "r"(a));
-  return v;
-}
-// A destination (dst: CTA << 24 | byte offset of the slot; -1: none) as an
-// address: of this CTA's shared memory, of another's, or none, so that the
-// stores on the chain are two predicated instructions and no branch.
-struct Slot {
-  unsigned a;
-  int near, far;
-};
-__device__ __forceinline__ Slot slot_of(unsigned smem, int rank, int dst) {
-  Slot s;
-  s.a = smem + (unsigned)(dst & 0xffffff);
-  s.near = dst >= 0 && (dst >> 24) == rank;
-  s.far = dst >= 0 && !s.near;
-  if (s.far) asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(s.a) : "r"(s.a), "r"(dst >> 24));
-  return s;
-}
-__device__ __forceinline__ void push(const Slot &s, float v) {
-  asm volatile("{ .reg .pred p, q; setp.ne.s32 p, %1, 0; setp.ne.s32 q, %2, 0; @p st.volatile.shared.f32 [%0], %3; "
-               "@q st.relaxed.cluster.shared::cluster.f32 [%0], %3; }" ::"r"(s.a), "r"(s.near), "r"(s.far), "f"(v)
-               : "memory");
-}
-__device__ __forceinline__ void push(const Slot &s, double v) {
-  asm volatile("{ .reg .pred p, q; setp.ne.s32 p, %1, 0; setp.ne.s32 q, %2, 0; @p st.volatile.shared.f64 [%0], %3; "
-               "@q st.relaxed.cluster.shared::cluster.f64 [%0], %3; }" ::"r"(s.a), "r"(s.near), "r"(s.far), "d"(v)
-               : "memory");
-}
 
 struct PushArgs {
   const int *wptr;  // groups of each warp of the cluster
@@ -152,17 +113,22 @@ __global__ void __launch_bounds__(32 * kPushW, 1) k_sptrsv_push(PushArgs A) {
     // the sums and the limit's tests inside, a poll took 0.13 us and a level of
     // a 64 x 64 grid 0.27 us).
     CT s[K];
-    for (int polls = 0, left = 1024;; --left) {
-      unsigned m = 0;
+    for (int polls = 0;;) {
+      bool ok = false;
 #pragma unroll
-      for (int t = 0; t < K; ++t) {
-        s[t] = ld_slot(a[t], (CT)0);
-        m = max(m, head(s[t]));
+      for (int u = 0; u < 4; ++u) {  // four polls between the limit's tests
+        unsigned m = 0;
+#pragma unroll
+        for (int t = 0; t < K; ++t) {
+          s[t] = ld_slot(a[t], (CT)0);
+          m = max(m, head(s[t]));
+        }
+        ok = __all_sync(0xffffffffu, m != 0xffffffffu);
+        if (ok) break;
       }
-      if (__all_sync(0xffffffffu, m != 0xffffffffu) || gave_up) break;
-      if (left == 0) {
-        left = 1024;
-        polls += 1024;
+      if (ok || gave_up) break;
+      polls += 4;
+      if ((polls & 1023) == 0) {
         if (polls > kMaxSpins && lane == 0) atomicOr(A.status, kStatusSpinTimeout);  // the solve is reported as failed
         gave_up = __any_sync(0xffffffffu, polls > kMaxSpins || (*(const volatile int *)A.status & kStatusSpinTimeout));
       }
@@ -309,7 +275,7 @@ int push_plan_host(const Pattern &T, bool lower, int bs, size_t ct, int C, PushH
     deg = std::max(deg, c);
     if (deg > (bs == 1 ? 8 : 4) || n >= 1 << 27) return 2;
   }
-  h.K = deg <= 3 ? 3 : deg <= 4 ? 4 : 8;
+  if (deg > h.K) h.K = deg <= 3 ? 3 : deg <= 4 ? 4 : 8;
   const int K = h.K;
   std::vector<int> lp(depth + 1, 0), rows(n);
   for (int i = 0; i < n; ++i) ++lp[lev[i] + 1];
