@@ -83,6 +83,10 @@ __global__ void __launch_bounds__(32 * kPushW, 1) k_sptrsv_push(PushArgs A) {
   // reads of earlier kernels is in place (the first one waited for them)
   if (!A.early) asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (A.done != nullptr && *(volatile const int *)A.done) {  // the same for every CTA
+    if (A.early) asm volatile("griddepcontrol.wait;" ::: "memory");
+    return;
+  }
   const int gb = A.wptr[rank * kPushW + warp], ge = A.wptr[rank * kPushW + warp + 1];
   // slot row 0 stays 0: the slots of the entries a row does not have
   for (unsigned k = threadIdx.x; k < A.fill; k += 32 * kPushW) {
@@ -94,7 +98,6 @@ __global__ void __launch_bounds__(32 * kPushW, 1) k_sptrsv_push(PushArgs A) {
   if (gb < ge) cur.load(A, gb, lane);
   cl.sync();  // every slot of the cluster is unsolved
   if (A.early) asm volatile("griddepcontrol.wait;" ::: "memory");
-  if (A.done != nullptr && *(volatile const int *)A.done) return;  // the same for every CTA
   bool gave_up = false;
   for (int g = gb; g < ge; ++g) {
     const int row = cur.rc < 0 ? -1 : (cur.rc & 0x7ffffff) * BS + comp, cnt = cur.rc < 0 ? 0 : cur.rc >> 27;
