@@ -127,15 +127,20 @@ struct lace_gpu_ctx {
   DBuf Arow, Acol, Aval;
   std::vector<int> hArow, hAcol;  // host copy of the resident CSR pattern
   int aval_version = 0;  // bumped whenever A's values change
-  // A in sliced ELL for the Arnoldi operator (CSR only): slice offsets, columns,
-  // source CSR entry of each slot (-1: padding) and the gathered values
-  DBuf sell_ptr, sell_col, sell_map, sell_val, sell_pair;
-  size_t sell_slots = 0;
-  bool sell_valid = false;
-  int sell_version = -1;
+  // A (and A^T) in sliced ELL for the Arnoldi operator (CSR only): slice
+  // offsets, columns, source CSR entry of each slot (-1: padding) and the
+  // gathered values
+  struct Sell {
+    DBuf ptr, col, map, val, pair;
+    size_t slots = 0;
+    bool valid = false;
+    int version = -1;
+  } sell, sell_t;
+  int build_sell(Sell &S, const int *row, const int *col, const int *src, bool pairs);
   int ensure_sell();
   // A^T for the adjoint
   bool AT_ready = false;
+  bool AT_pattern = false;  // ATrow, ATcol, map_at2a and sell_t belong to the resident pattern
   DBuf ATrow, ATcol, ATval, map_at2a;
 
   // factor patterns and maps
