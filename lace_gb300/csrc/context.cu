@@ -717,7 +717,7 @@ extern "C" int lace_gpu_ctx_create(lace_gpu_ctx **out, int device, void *stream)
   cudaMemsetAsync(c->ctrl_buf.p, 0, sizeof(Control) * 2, c->stream);
   cudaMemsetAsync(c->cycle_buf.p, 0, sizeof(Cycle), c->stream);
   cudaMemsetAsync(c->cnt_buf.p, 0, 64 * sizeof(int), c->stream);
-  if (cudaMallocHost(&c->h_ctrl, sizeof(Control)) != cudaSuccess ||
+  if (cudaMallocHost(&c->h_ctrl, sizeof(Control) + 2 * sizeof(int)) != cudaSuccess ||
       cudaMallocHost(&c->h_scal, kScalHost * sizeof(double)) != cudaSuccess) {
     delete c;
     return set_err(DEV_ERR_HOST_ALLOC);
@@ -726,11 +726,18 @@ extern "C" int lace_gpu_ctx_create(lace_gpu_ctx **out, int device, void *stream)
     delete c;
     return set_err(DEV_ERR_UNKNOWN);
   }
+  c->h_done = (int *)(c->h_ctrl + 1);
   *out = c;
   return DEV_SUCCESS;
 }
 
 lace_gpu_ctx::~lace_gpu_ctx() {
+  if (poll) {
+    cudaStreamSynchronize(poll);
+    cudaStreamDestroy(poll);
+  }
+  for (cudaEvent_t e : {seg_end[0], seg_end[1], seg_read[0], seg_read[1]})
+    if (e) cudaEventDestroy(e);
   for (auto &kv : graphs) cudaGraphExecDestroy(kv.second);
   graphs.clear();
   if (h_ctrl) cudaFreeHost(h_ctrl);
@@ -2217,9 +2224,9 @@ ArnoldiArgs lace_gpu_ctx::arnoldi_args(int m, bool adjoint) {
 }
 
 // the search-direction loop of one cycle (LACE :311-759), all on the device
-int lace_gpu_ctx::enqueue_cycle_body(const ArnoldiArgs &a, int m, bool adjoint, bool capturing) {
+int lace_gpu_ctx::enqueue_cycle_body(const ArnoldiArgs &a, int j0, int j1, bool adjoint, bool capturing) {
   const int t1 = adjoint ? 2 : 0, t2 = adjoint ? 3 : 1;
-  for (int j = 0; j < m; ++j) {
+  for (int j = j0; j < j1; ++j) {
     void *zj = (char *)a.Z + (size_t)j * a.ldz * (a.z_f32 ? 4 : 8);
     // both outputs were marked unsolved by the kernel before (a.prefill)
     int rc = solve_pair(t1, t2, a.q, a.q_f32, zj, a.z_f32, true, a.prefill != 0);
@@ -2248,10 +2255,10 @@ int lace_gpu_ctx::enqueue_cycle_body(const ArnoldiArgs &a, int m, bool adjoint, 
 
 // the modified Gram-Schmidt search-direction loop of one cycle
 // (src/fgmres_restart.cpp:227-494), all on the device
-int lace_gpu_ctx::enqueue_mgs_body(const ArnoldiArgs &a, int m, bool capturing) {
+int lace_gpu_ctx::enqueue_mgs_body(const ArnoldiArgs &a, int j0, int j1, bool capturing) {
   // LACE's test reorthogonalises for reorth 0 (when needed) and 2 (always)
   const bool second = a.mgs_reorth == 0 || a.mgs_reorth == 2;
-  for (int j = 0; j < m; ++j) {
+  for (int j = j0; j < j1; ++j) {
     void *zj = (char *)a.Z + (size_t)j * a.ldz * (a.z_f32 ? 4 : 8);
     const double *vj = a.V + (size_t)j * a.ldv;
     // z_j = U^{-1} L^{-1} v_j (:239-270); outputs marked unsolved before
@@ -2348,6 +2355,13 @@ int lace_gpu_ctx::fgmres(const double *b, double *x, int m, int restart_max, int
   if (!rc && cudaStreamSynchronize(stream) != cudaSuccess) rc = DEV_ERR_UNKNOWN;
   if (rc) return rc;
   sc.mark("solve plans");
+  if (!poll) {
+    if (cudaStreamCreateWithFlags(&poll, cudaStreamNonBlocking) != cudaSuccess) return DEV_ERR_UNKNOWN;
+    for (int k = 0; k < 2; ++k)
+      if (cudaEventCreateWithFlags(&seg_end[k], cudaEventDisableTiming) != cudaSuccess ||
+          cudaEventCreateWithFlags(&seg_read[k], cudaEventDisableTiming) != cudaSuccess)
+        return DEV_ERR_UNKNOWN;
+  }
   if (mgs && !side && cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking) != cudaSuccess)
     return DEV_ERR_UNKNOWN;
   ArnoldiArgs a = arnoldi_args(m, adjoint);
@@ -2366,15 +2380,13 @@ int lace_gpu_ctx::fgmres(const double *b, double *x, int m, int restart_max, int
     int zero = 0;
     LCHK(cudaMemcpyAsync(&a.ctrl->status, &zero, 4, cudaMemcpyHostToDevice, stream));
   }
-  const auto key = std::make_tuple(m, adjoint ? 1 : 0, opt.trsv_mode, rows_per_lane,
-                                   opt.jacobi_sweeps, (int)vtype(), opt.monitor_orthog, lanes, method,
-                                   mgs ? (restarted ? 1 : 0) : 0, mgs ? reorth : 0);
   int total = 0;
   bool converged = false;
   int last_cycle = 0, last_steps = 0;
   last_reorth = 0;
   last_orth.clear();
-  double rnorm0 = 0.0, final_res = 0.0;
+  double rnorm0 = 0.0, final_res = 0.0, cycle_res = 0.0;  // cycle_res: where the cycle started
+  double expected = 0.0;  // directions still needed, at the last cycle's rate
   for (int restart = 0; restart < restart_max; ++restart) {
     launch_cycle_residual(stream, a, b, x, mgs);
     if (mgs) {
@@ -2384,43 +2396,67 @@ int lace_gpu_ctx::fgmres(const double *b, double *x, int m, int restart_max, int
       if (opt.monitor_orthog && Qmon.p)
         launch_convert(stream, n, a.q_f32 ? VType::F32 : VType::F64, a.q, VType::F64, Qmon.p);
     }
-    if (opt.use_graph) {
-      auto it = graphs.find(key);
-      if (it == graphs.end()) {
-        SetupClock gc(verbose);
-        cudaGraphExec_t ge = nullptr;
-        for (int attempt = 0; attempt < 3 && !ge; ++attempt) {
-          cudaGraph_t g;
-          LCHK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-          rc = mgs ? enqueue_mgs_body(a, m, true) : enqueue_cycle_body(a, m, adjoint, true);
-          cudaError_t ce = cudaStreamEndCapture(stream, &g);
-          if (rc == DEV_ERR_NOT_SUPPORTED && attempt < 2) {
-            // a refused cooperative launch or conditional node (the flag
-            // that chose it is cleared): capture again without it
-            if (ce == cudaSuccess) cudaGraphDestroy(g);
-            cudaGetLastError();
-            if (verbose && !cond_nodes) printf("%% conditional graph nodes unavailable: the second Gram-Schmidt pass launches always\n");
-            rc = 0;
-            continue;
+    // The cycle in segments of kSegment directions.  A direction past the last
+    // one needed only costs its launches (2-4 us a kernel), but a whole cycle of
+    // them was 0.3 ms of a solve that converges in 5 of 30 directions.  So the
+    // host stops after a segment that ended the cycle: it reads the flag on
+    // a stream of its own while the next segment runs.  A segment starts 4 us
+    // late, so a cycle that the last one's rate lets run to its end is one (64^2
+    // with Gram-Schmidt, five cycles: 2 % slower all in segments).
+    const int seg = expected >= m ? m : kSegment, nseg = (m + seg - 1) / seg;
+    for (int s = 0; s < nseg; ++s) {
+      const int j0 = s * seg, j1 = std::min(m, j0 + seg);
+      if (opt.use_graph) {
+        const auto key = std::make_tuple(m, adjoint ? 1 : 0, opt.trsv_mode, rows_per_lane, opt.jacobi_sweeps,
+                                         (int)vtype(), opt.monitor_orthog, lanes, method,
+                                         mgs ? (restarted ? 1 : 0) : 0, mgs ? reorth : 0, seg == m ? -1 : s);
+        auto it = graphs.find(key);
+        if (it == graphs.end()) {
+          SetupClock gc(verbose);
+          cudaGraphExec_t ge = nullptr;
+          for (int attempt = 0; attempt < 3 && !ge; ++attempt) {
+            cudaGraph_t g;
+            LCHK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
+            rc = mgs ? enqueue_mgs_body(a, j0, j1, true) : enqueue_cycle_body(a, j0, j1, adjoint, true);
+            cudaError_t ce = cudaStreamEndCapture(stream, &g);
+            if (rc == DEV_ERR_NOT_SUPPORTED && attempt < 2) {
+              // a refused cooperative launch or conditional node (the flag
+              // that chose it is cleared): capture again without it
+              if (ce == cudaSuccess) cudaGraphDestroy(g);
+              cudaGetLastError();
+              if (verbose && !cond_nodes) printf("%% conditional graph nodes unavailable: the second Gram-Schmidt pass launches always\n");
+              rc = 0;
+              continue;
+            }
+            if (rc) {
+              if (ce == cudaSuccess) cudaGraphDestroy(g);
+              return rc;
+            }
+            LCHK(ce);
+            gc.mark("cycle graph capture");
+            ce = cudaGraphInstantiate(&ge, g, 0);
+            cudaGraphDestroy(g);
+            LCHK(ce);
+            gc.mark("cycle graph instantiation");
           }
-          if (rc) {
-            if (ce == cudaSuccess) cudaGraphDestroy(g);
-            return rc;
-          }
-          LCHK(ce);
-          gc.mark("cycle graph capture");
-          ce = cudaGraphInstantiate(&ge, g, 0);
-          cudaGraphDestroy(g);
-          LCHK(ce);
-          gc.mark("cycle graph instantiation");
+          if (!ge) return DEV_ERR_UNKNOWN;
+          it = graphs.emplace(key, ge).first;
         }
-        if (!ge) return DEV_ERR_UNKNOWN;
-        it = graphs.emplace(key, ge).first;
+        LCHK(cudaGraphLaunch(it->second, stream));
+      } else {
+        rc = mgs ? enqueue_mgs_body(a, j0, j1, false) : enqueue_cycle_body(a, j0, j1, adjoint, false);
+        if (rc) return rc;
       }
-      LCHK(cudaGraphLaunch(it->second, stream));
-    } else {
-      rc = mgs ? enqueue_mgs_body(a, m, false) : enqueue_cycle_body(a, m, adjoint, false);
-      if (rc) return rc;
+      if (s + 1 < nseg) {
+        LCHK(cudaEventRecord(seg_end[s & 1], stream));
+        LCHK(cudaStreamWaitEvent(poll, seg_end[s & 1], 0));
+        LCHK(cudaMemcpyAsync(h_done + (s & 1), &a.ctrl->done, 4, cudaMemcpyDeviceToHost, poll));
+        LCHK(cudaEventRecord(seg_read[s & 1], poll));
+        if (s > 0) {
+          LCHK(cudaEventSynchronize(seg_read[(s - 1) & 1]));
+          if (h_done[(s - 1) & 1]) break;
+        }
+      }
     }
     if (mgs) launch_mgs_xupdate(stream, a, x);
     else launch_xupdate(stream, a, x);
@@ -2468,6 +2504,9 @@ int lace_gpu_ctx::fgmres(const double *b, double *x, int m, int restart_max, int
     }
     if (hc.status & kStatusBreakdown) break;
     if (ns == 0) break;
+    if (restart == 0) cycle_res = hc.rnorm0;
+    expected = final_res < cycle_res ? ns * std::log(final_res / hc.rtol_abs) / std::log(cycle_res / final_res) : m;
+    cycle_res = final_res;
     int zero = 0;
     LCHK(cudaMemcpyAsync(&cy->first_cycle, &zero, 4, cudaMemcpyHostToDevice, stream));
   }

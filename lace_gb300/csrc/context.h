@@ -207,7 +207,13 @@ struct lace_gpu_ctx {
   DBuf dropin_b, dropin_x;  // right-hand side and solution of the drop-in FGMRES
   lace::Control *h_ctrl = nullptr;
   double *h_scal = nullptr;
-  std::map<std::tuple<int, int, int, int, int, int, int, int, int, int, int>, cudaGraphExec_t> graphs;
+  // captured segments of a cycle
+  std::map<std::tuple<int, int, int, int, int, int, int, int, int, int, int, int>, cudaGraphExec_t> graphs;
+  static constexpr int kSegment = 4;  // directions
+  // where the host reads whether a segment ended the cycle
+  cudaStream_t poll = nullptr;
+  cudaEvent_t seg_end[2] = {nullptr, nullptr}, seg_read[2] = {nullptr, nullptr};
+  int *h_done = nullptr;
   // second stream: the body of the conditional Gram-Schmidt second pass is
   // captured on it
   cudaStream_t side = nullptr;
@@ -267,10 +273,11 @@ struct lace_gpu_ctx {
   int ensure_krylov(int m, bool monitor);
   int ensure_AT();
   lace::ArnoldiArgs arnoldi_args(int m, bool adjoint);
-  int enqueue_cycle_body(const lace::ArnoldiArgs &a, int m, bool adjoint, bool capturing);
+  // directions j0 to j1 - 1 of a cycle
+  int enqueue_cycle_body(const lace::ArnoldiArgs &a, int j0, int j1, bool adjoint, bool capturing);
   // the modified Gram-Schmidt cycle; capturing: inside a stream capture (the
   // second pass goes into conditional nodes when cond_nodes)
-  int enqueue_mgs_body(const lace::ArnoldiArgs &a, int m, bool capturing);
+  int enqueue_mgs_body(const lace::ArnoldiArgs &a, int j0, int j1, bool capturing);
   // method 0: Householder (fgmres_householder_restart.cpp); 1: modified
   // Gram-Schmidt, restarted (fgmres_restart.cpp) or one cycle (fgmres.cpp)
   // with reorth as LACE's gmres_par->reorth
