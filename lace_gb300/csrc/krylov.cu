@@ -586,6 +586,31 @@ __global__ void __launch_bounds__(kTPB) k_passC(int n, double *__restrict__ V, f
 constexpr int kHHTPB = 1024;
 constexpr int kHHSmemMax = 200 * 1024;  // rows of w per block: at most 25,600
 
+// the small matrices of steps 0..j (and rows 0..j+1 of the reflectors) into L1,
+// ahead of the sums that read them entry by entry between the grid's folds
+__device__ __forceinline__ void prefetch_l1(const void *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+__device__ __forceinline__ void hh_prefetch(const double *M, int jp1) {
+  // a line is 16 entries of a column
+  for (int e = threadIdx.x; e < jp1 * ((jp1 + 15) >> 4); e += blockDim.x)
+    prefetch_l1(M + (size_t)(e % jp1) * kLdT + 16 * (e / jp1));
+}
+
+// sums of f(k, l) over l in [first(k), last(k)) for k < count, four threads an
+// entry (whole warps: a warp's butterfly costs 5 FP64 additions an entry, of 16
+// cycles each, and leaves most lanes without a term); done(k, sum) by one of them
+template <typename First, typename Last, typename F, typename Done>
+__device__ __forceinline__ void quad_sums(int count, First first, Last last, F f, Done done) {
+  for (int e = threadIdx.x; e < 4 * ((count + 7) & ~7); e += blockDim.x) {
+    const int k = e >> 2;
+    double t = 0.0;
+    if (k < count)
+      for (int l = first(k) + (e & 3); l < last(k); l += 4) t = f(k, l, t);
+    t += __shfl_xor_sync(0xffffffffu, t, 1);
+    t += __shfl_xor_sync(0xffffffffu, t, 2);
+    if (k < count && (e & 3) == 0) done(k, t);
+  }
+}
+
 struct HHStep {
   int n, rb;
   OpView op;  // sliced ELL
@@ -600,6 +625,50 @@ struct HHStep {
   int m;
   Prefill pf;
 };
+
+// The Hessenberg column j (rows 0..j of w, -dd below), its Givens rotation and
+// the convergence test (LACE :658-714 and opt4's non-finite stop), by the block
+// that calls it; s_: 768 doubles
+__device__ __forceinline__ void hh_rotate(const HHStep &a, int j, double dd, const double *wtop, double *s_) {
+  Cycle *cy = a.cy;
+  const int lane = threadIdx.x & 31, jp1 = j + 1;
+  double *sh = s_, *scs = s_ + 256, *ssn = s_ + 512;
+  if (threadIdx.x < 32) {
+    for (int k = lane; k <= j; k += 32) sh[k] = wtop[k];
+    for (int k = lane; k < j; k += 32) {
+      scs[k] = cy->cs[k];
+      ssn[k] = cy->sn[k];
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int k = 0; k < j; ++k) {
+      const double t0 = sh[k], t1 = sh[k + 1];
+      sh[k + 1] = -ssn[k] * t0 + scs[k] * t1;
+      sh[k] = scs[k] * t0 + ssn[k] * t1;
+    }
+    double c, sn;
+    givens_rot(sh[j], -dd, 4.9406564584124654e-324, &c, &sn);
+    cy->cs[j] = c;
+    cy->sn[j] = sn;
+    sh[j] = c * sh[j] - sn * dd;
+    const double gj = cy->g[j];
+    cy->g[jp1] = -sn * gj;
+    cy->g[j] = c * gj;
+    const double resid = fabs(-sn * gj);
+    cy->hist[j] = resid;
+    a.ctrl->resid = resid;
+    const bool conv = resid < a.ctrl->rtol_abs;
+    double *R = cy->R + (size_t)j * kLdT;
+    for (int k = 0; k <= j; ++k) R[k] = sh[k];
+    if (conv || j == a.m - 1 || !(resid == resid)) {
+      a.ctrl->nsteps = jp1;
+      a.ctrl->converged = conv ? 1 : 0;
+      if (!(resid == resid)) a.ctrl->status |= kStatusBreakdown;
+      a.ctrl->done = 1;
+    }
+  }
+}
 
 template <typename ZT, typename QT>
 __global__ void __launch_bounds__(kHHTPB, 1) k_hh_step(HHStep a, int j) {
@@ -621,6 +690,7 @@ __global__ void __launch_bounds__(kHHTPB, 1) k_hh_step(HHStep a, int j) {
   const size_t ldv = a.ldv;
   const double *__restrict__ V = a.V;
   Cycle *cy = a.cy;
+  hh_prefetch(cy->T, jp1);
   // ---- pass A: w = A z_j (a warp per 32-row slice), s = V^T w
   {
     const ZT *z = (const ZT *)a.z;
@@ -656,11 +726,9 @@ __global__ void __launch_bounds__(kHHTPB, 1) k_hh_step(HHStep a, int j) {
   hh_block_dots(V, ldv, jp1, r0, r1, -1, sw, swarp, sacc);
   if (!hh_grid_fold(sacc, jp1, a.fold, tag, a.ctrl, sres)) return;
   // y = T^T s
-  for (int k = threadIdx.x; k < jp1; k += T) {
-    double y = 0.0;
-    for (int l = 0; l <= k; ++l) y = fma(cy->T[l + k * kLdT], sres[l], y);
-    sy[k] = y;
-  }
+  quad_sums(jp1, [](int) { return 0; }, [](int k) { return k + 1; },
+            [&](int k, int l, double t) { return fma(cy->T[l + k * kLdT], sres[l], t); },
+            [&](int k, double t) { sy[k] = t; });
   __syncthreads();
   // ---- pass B: w -= V y (a row pair per thread), then V^T w over rows > j
   // and ||w_{j+1:}||^2; rows 0..j+1 of w published for every block
@@ -724,20 +792,18 @@ __global__ void __launch_bounds__(kHHTPB, 1) k_hh_step(HHStep a, int j) {
   if (threadIdx.x == 0) srho[jp1] = s_vjj;
   __syncthreads();
   // the new column of T (kept in sacc) and c
-  for (int k = threadIdx.x; k < jp1; k += T) {
-    double t = 0.0;
-    for (int l = k; l < jp1; ++l) t = fma(cy->T[k + l * kLdT], sd[l], t);
-    sacc[k] = -2.0 * t;
-  }
+  quad_sums(jp1, [](int k) { return k; }, [&](int) { return jp1; },
+            [&](int k, int l, double t) { return fma(cy->T[k + l * kLdT], sd[l], t); },
+            [&](int k, double t) { sacc[k] = -2.0 * t; });
   if (threadIdx.x == 0) sacc[jp1] = 2.0;
   __syncthreads();
-  for (int k = threadIdx.x; k <= jp1; k += T) {
-    double t = 0.0;
-    for (int l = k; l < jp1; ++l) t = fma(cy->T[k + l * kLdT], srho[l], t);
-    t = fma(sacc[k], srho[jp1], t);
-    sc[k] = t;
-    scf[k] = (float)t;
-  }
+  quad_sums(jp1 + 1, [](int k) { return k; }, [&](int) { return jp1; },
+            [&](int k, int l, double t) { return fma(cy->T[k + l * kLdT], srho[l], t); },
+            [&](int k, double t) {
+              t = fma(sacc[k], srho[jp1], t);
+              sc[k] = t;
+              scf[k] = (float)t;
+            });
   __syncthreads();
   if (blockIdx.x == 0) {
     // the record: T column, reflector scalars, c; rotations and the test
@@ -747,35 +813,6 @@ __global__ void __launch_bounds__(kHHTPB, 1) k_hh_step(HHStep a, int j) {
     if (threadIdx.x == 0) {
       cy->dd = s_dd;
       cy->inv_alpha = s_ia;
-      // Hessenberg column j: h_k = w_k (k <= j), h_{j+1} = -dd (LACE :658-701)
-      double *sh = sbuf;
-      for (int k = 0; k <= j; ++k) sh[k] = wtop[k];
-      for (int k = 0; k < j; ++k) {
-        const double t0 = sh[k], t1 = sh[k + 1];
-        sh[k + 1] = -cy->sn[k] * t0 + cy->cs[k] * t1;
-        sh[k] = cy->cs[k] * t0 + cy->sn[k] * t1;
-      }
-      const double dd = s_dd;
-      double c, sn;
-      givens_rot(sh[j], -dd, 4.9406564584124654e-324, &c, &sn);
-      cy->cs[j] = c;
-      cy->sn[j] = sn;
-      sh[j] = c * sh[j] - sn * dd;
-      const double gj = cy->g[j];
-      cy->g[jp1] = -sn * gj;
-      cy->g[j] = c * gj;
-      const double resid = fabs(-sn * gj);
-      cy->hist[j] = resid;
-      a.ctrl->resid = resid;
-      const bool conv = resid < a.ctrl->rtol_abs;
-      double *R = cy->R + (size_t)j * kLdT;
-      for (int k = 0; k <= j; ++k) R[k] = sh[k];
-      if (conv || j == a.m - 1 || !(resid == resid)) {  // LACE :714 (+ opt4's non-finite stop)
-        a.ctrl->nsteps = jp1;
-        a.ctrl->converged = conv ? 1 : 0;
-        if (!(resid == resid)) a.ctrl->status |= kStatusBreakdown;
-        a.ctrl->done = 1;
-      }
     }
   }
   // ---- pass C: v_{j+1} and q = e_{j+1} - V_{j+1} c for this block's rows
@@ -811,6 +848,9 @@ __global__ void __launch_bounds__(kHHTPB, 1) k_hh_step(HHStep a, int j) {
     q[i] = (QT)(((i == jp1 ? 1.0 : 0.0) - v * sc[jp1]) - vcomb8(V, ldv, i, jp1, sc));
     prefill_row(a.pf, i);
   }
+  __syncthreads();  // sbuf
+  // in the last block, which has the fewest rows
+  if (blockIdx.x == gridDim.x - 1) hh_rotate(a, j, dd, wtop, sbuf);
 }
 
 // --------------------------- the one-kernel step in double-float arithmetic
@@ -1071,6 +1111,8 @@ __global__ void __launch_bounds__(kHHTPB, 1) k_hh_step_df(HHStepDF ad, int j) {
   const float *__restrict__ Vlo = ad.Vlo;
   Cycle *cy = a.cy;
   const int G = gridDim.x;
+  hh_prefetch(cy->T, jp1);
+  hh_prefetch(cy->G, jp1);
   // g's block partials from the previous step, folded with s below
   for (int k = threadIdx.x; k < j; k += T) sacc[jp1 + k] = __ldcg(&ad.carry[(size_t)k * G + blockIdx.x]);
   // ---- pass A: w = A z_j in pair arithmetic (the operator's values as
@@ -1109,30 +1151,24 @@ __global__ void __launch_bounds__(kHHTPB, 1) k_hh_step_df(HHStepDF ad, int j) {
   __syncthreads();
   hh_block_dots_df(Vf, Vlo, ldv, jp1, r0, r1, -1, DfShared{swd}, swarp, sacc);
   if (!hh_grid_fold(sacc, jp1 + j, a.fold, tag, a.ctrl, sres)) return;
-  // T(:, j) = [-2 T_j g ; 2] and G(:, j) = [g ; 1] (a warp per entry)
-  for (int k = wid; k <= j; k += nw) {
-    double t = 0.0;
-    for (int l = k + lane; l < j; l += 32) t = fma(cy->T[k + l * kLdT], sres[jp1 + l], t);
-    t = warp_sum(t);
-    if (lane == 0) {
-      stc[k] = k < j ? -2.0 * t : 2.0;
-      sg[k] = k < j ? sres[jp1 + k] : 1.0;
-    }
-  }
+  // T(:, j) = [-2 T_j g ; 2] and G(:, j) = [g ; 1] 
+  quad_sums(jp1, [](int k) { return k; }, [&](int) { return j; },
+            [&](int k, int l, double t) { return fma(cy->T[k + l * kLdT], sres[jp1 + l], t); },
+            [&](int k, double t) {
+              stc[k] = k < j ? -2.0 * t : 2.0;
+              sg[k] = k < j ? sres[jp1 + k] : 1.0;
+            });
   __syncthreads();
   // y = T^T s, as a pair (and in FP64); s kept for the second dot set
-  for (int k = wid; k < jp1; k += nw) {
-    double t = 0.0;
-    for (int l = lane; l <= k; l += 32) t = fma(k < j ? cy->T[l + k * kLdT] : stc[l], sres[l], t);
-    t = warp_sum(t);
-    if (lane == 0) {
-      const float2 d = df_split(t);
-      syh[k] = d.x;
-      syl[k] = d.y;
-      sy[k] = t;
-      ss[k] = sres[k];
-    }
-  }
+  quad_sums(jp1, [](int) { return 0; }, [](int k) { return k + 1; },
+            [&](int k, int l, double t) { return fma(k < j ? cy->T[l + k * kLdT] : stc[l], sres[l], t); },
+            [&](int k, double t) {
+              const float2 d = df_split(t);
+              syh[k] = d.x;
+              syl[k] = d.y;
+              sy[k] = t;
+              ss[k] = sres[k];
+            });
   if (blockIdx.x == 0) {  // read by the later steps only
     for (int k = threadIdx.x; k < kLdT; k += T) cy->T[k + j * kLdT] = k <= j ? stc[k] : 0.0;
     for (int k = threadIdx.x; k <= j; k += T) {
@@ -1187,17 +1223,14 @@ __global__ void __launch_bounds__(kHHTPB, 1) k_hh_step_df(HHStepDF ad, int j) {
   const double nrm2 = jp1 < n ? sres[0] : 0.0;
   // V^T w over rows > j after the update, without a pass over V:
   // s - G y over all rows, less the rows <= j that their owners published
-  for (int k = wid; k < jp1; k += nw) {
-    double t = 0.0;
-    for (int l = lane; l < jp1; l += 32) {
-      const double gkl = l == j ? sg[k] : (k == j ? sg[l] : cy->G[k + l * kLdT]);
-      t = fma(gkl, sy[l], t);
-    }
-    for (int i = k + lane; i <= j; i += 32) t = fma(a.V[(size_t)k * ldv + i], wtop[i], t);
-    t = warp_sum(t);
-    if (lane == 0) s2[k] = ss[k] - t;
-  }
-  if (threadIdx.x == 0) {
+  quad_sums(jp1, [](int) { return 0; }, [&](int) { return jp1; },
+            [&](int k, int l, double t) {
+              const double gkl = l == j ? sg[k] : (k == j ? sg[l] : cy->G[k + l * kLdT]);
+              t = fma(gkl, sy[l], t);
+              return l >= k ? fma(a.V[(size_t)k * ldv + l], wtop[l], t) : t;
+            },
+            [&](int k, double t) { s2[k] = ss[k] - t; });
+  if (threadIdx.x == T - 1) {
     const double wn = sqrt(nrm2);
     const double wj1 = jp1 < n ? wtop[jp1] : 0.0;
     const double dd = mysgn(wj1) * wn;
@@ -1216,24 +1249,18 @@ __global__ void __launch_bounds__(kHHTPB, 1) k_hh_step_df(HHStepDF ad, int j) {
   if (threadIdx.x == 0) srho[jp1] = s_vjj;
   __syncthreads();
   // T's column j+1 (provisional, see above), then c = T_{j+1} rho
-  for (int k = wid; k < jp1; k += nw) {
-    double t = 0.0;
-    for (int l = k + lane; l <= j; l += 32) t = fma(l == j ? stc[k] : cy->T[k + l * kLdT], sd[l], t);
-    t = warp_sum(t);
-    if (lane == 0) sacc[k] = -2.0 * t;
-  }
+  quad_sums(jp1, [](int k) { return k; }, [&](int) { return jp1; },
+            [&](int k, int l, double t) { return fma(l == j ? stc[k] : cy->T[k + l * kLdT], sd[l], t); },
+            [&](int k, double t) { sacc[k] = -2.0 * t; });
   if (threadIdx.x == 0) sacc[jp1] = 2.0;
   __syncthreads();
-  for (int k = wid; k <= jp1; k += nw) {
-    double t = 0.0;
-    for (int l = k + lane; l <= j; l += 32) t = fma(l == j ? stc[k] : cy->T[k + l * kLdT], srho[l], t);
-    t = warp_sum(t);
-    if (lane == 0) {
-      t = fma(sacc[k], srho[jp1], t);
-      sc[k] = t;
-      scf[k] = (float)t;
-    }
-  }
+  quad_sums(jp1 + 1, [](int k) { return k; }, [&](int) { return jp1; },
+            [&](int k, int l, double t) { return fma(l == j ? stc[k] : cy->T[k + l * kLdT], srho[l], t); },
+            [&](int k, double t) {
+              t = fma(sacc[k], srho[jp1], t);
+              sc[k] = t;
+              scf[k] = (float)t;
+            });
   __syncthreads();
   if (blockIdx.x == 0) {
     double *Tg = cy->T;
@@ -1283,46 +1310,8 @@ __global__ void __launch_bounds__(kHHTPB, 1) k_hh_step_df(HHStepDF ad, int j) {
   __syncthreads();
   hh_passC_rows(Vf, Vlo, ldv, jp1, r0, r1, jp1, swd, scf, (float *)a.q, reinterpret_cast<float2 *>(sbuf), sg);
   for (int k = threadIdx.x; k < jp1; k += T) ad.carry[(size_t)k * G + blockIdx.x] = sg[k];
-  // ---- the Hessenberg column j (rows 0..j of w, -dd below), its Givens
-  // rotation and the convergence test, in the last block (the fewest rows)
-  if (blockIdx.x == G - 1) {
-    double *sh = sbuf, *scs = sbuf + 256, *ssn = sbuf + 512;
-    if (wid == 0) {
-      for (int k = lane; k <= j; k += 32) sh[k] = wtop[k];
-      for (int k = lane; k < j; k += 32) {
-        scs[k] = cy->cs[k];
-        ssn[k] = cy->sn[k];
-      }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      for (int k = 0; k < j; ++k) {
-        const double t0 = sh[k], t1 = sh[k + 1];
-        sh[k + 1] = -ssn[k] * t0 + scs[k] * t1;
-        sh[k] = scs[k] * t0 + ssn[k] * t1;
-      }
-      double c, sn;
-      givens_rot(sh[j], -dd, 4.9406564584124654e-324, &c, &sn);
-      cy->cs[j] = c;
-      cy->sn[j] = sn;
-      sh[j] = c * sh[j] - sn * dd;
-      const double gj = cy->g[j];
-      cy->g[jp1] = -sn * gj;
-      cy->g[j] = c * gj;
-      const double resid = fabs(-sn * gj);
-      cy->hist[j] = resid;
-      a.ctrl->resid = resid;
-      const bool conv = resid < a.ctrl->rtol_abs;
-      double *R = cy->R + (size_t)j * kLdT;
-      for (int k = 0; k <= j; ++k) R[k] = sh[k];
-      if (conv || j == a.m - 1 || !(resid == resid)) {
-        a.ctrl->nsteps = jp1;
-        a.ctrl->converged = conv ? 1 : 0;
-        if (!(resid == resid)) a.ctrl->status |= kStatusBreakdown;
-        a.ctrl->done = 1;
-      }
-    }
-  }
+  // in the last block, which has the fewest rows
+  if (blockIdx.x == gridDim.x - 1) hh_rotate(a, j, dd, wtop, sbuf);
 }
 
 // ----------------------------------------------- orthogonality monitor
