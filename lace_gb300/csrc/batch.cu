@@ -9,8 +9,8 @@
 // (system, rhs) pair - as one persistent launch, captured in a CUDA graph when
 // the context's options ask for graphs: a cluster of CTAs per pair
 // (batch_cluster.cu), or, where a system's triangles do not fit a cluster's
-// shared memory, a CTA per system and up to four of its right-hand sides
-// (batch_persist.cu).
+// shared memory or the jobs fill the chip anyway, a CTA per system and up to four
+// of its right-hand sides (batch_persist.cu).
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -46,6 +46,8 @@ struct lace_gpu_batch {
 };
 
 namespace {
+
+constexpr int kSplitRows = 16384;  // single-CTA form: systems from here on give each right-hand side its own job
 
 // levels of one triangle of system rows [r0, r0 + n) (global indices in
 // the block-diagonal CSR): lower: a row's level is one more than the largest
@@ -190,7 +192,6 @@ extern "C" int lace_gpu_batch_create(lace_gpu_batch **out, lace_gpu_ctx *ctx, in
   // SMs: the longest of them sets the launch's time), a smaller one takes its
   // right-hand sides in groups of up to four (the operator, factor and
   // level-barrier work shared)
-  constexpr int kSplitRows = 16384;
   std::vector<int> order(nsys);
   std::iota(order.begin(), order.end(), 0);
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return n[a] > n[b]; });
@@ -245,8 +246,27 @@ static double cluster_cost(const lace_gpu_batch *B, const std::vector<int> &leve
   return std::max(top, sum / std::max(1, num_sms() / C));
 }
 
+// The same of the single-CTA form: per direction 16.5 ns a row and right-hand
+// side and 0.72 us a level, its right-hand sides in lockstep, one job an SM.  It
+// stays the better one where the jobs fill the chip (a level's barrier serves four
+// right-hand sides): 256 systems of 1,024 to 65,536 rows, four right-hand sides,
+// 3.6 s against 5.2 on clusters; the 24 systems above 252 ms against 37.
+static double persist_cost(const lace_gpu_batch *B, const std::vector<int> &levels) {
+  double sum = 0.0, top = 0.0;
+  for (int s = 0; s < B->nsys; ++s) {
+    const int g = B->n[s] >= kSplitRows ? 1 : batch_persist_rhs();
+    for (int r = 0; r < B->nrhs; r += g) {
+      const double t =
+          std::sqrt((double)B->n[s]) * (0.0165 * B->n[s] * std::min(g, B->nrhs - r) + 0.72 * levels[s] + 10.0);
+      sum += t;
+      top = std::max(top, t);
+    }
+  }
+  return std::max(top, sum / std::max(1, num_sms()));
+}
+
 // The cluster form's plans for value size ct and m directions (C = 0: the
-// batch does not fit it).
+// batch does not fit it, or the single-CTA form is the better one).
 static int cluster_plan(lace_gpu_batch *B, int m, size_t ct) {
   if (B->plan_ct == (int)ct && B->m == m) return 0;
   B->C = 0;
@@ -303,11 +323,17 @@ static int cluster_plan(lace_gpu_batch *B, int m, size_t ct) {
   std::vector<int> order{1, 2, 4, 8};
   std::stable_sort(order.begin(), order.end(),
                    [&](int a, int b) { return cluster_cost(B, levels, a) < cluster_cost(B, levels, b); });
+  const double other = persist_cost(B, levels);
   for (int C : order) {
+    if (cluster_cost(B, levels, C) >= other) break;
     int rb = 0;
     const size_t rest = batch_cluster_smem(0, B->nmax, m, C, &rb);
     if (rest + 1024 > batch_cluster_smem_max()) continue;
     const size_t cap = batch_cluster_smem_max() - rest;
+    size_t most = 0;  // slots of the largest triangle, without the groups' padding
+    for (auto &y : S)
+      for (auto &T : y.T) most = std::max(most, T.idx.size() - (size_t)T.n);
+    if (most * ct > cap * C) continue;
     int K = 2;
     for (bool again = true; again;) {
       again = false;

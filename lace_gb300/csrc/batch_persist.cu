@@ -1,4 +1,5 @@
-// Batched solves as one persistent launch: every CTA takes systems from a
+// Batched solves whose systems fit no cluster, or are enough to fill the chip
+// (batch_cluster.cu takes the others), as one persistent launch: every CTA takes systems from a
 // queue (largest first) and carries each through ParILU(0) and FGMRES-
 // Householder for all of its right-hand sides (four in lockstep) on its own,
 // with CTA barriers only - no grid barrier, no wait on another CTA.

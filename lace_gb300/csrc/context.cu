@@ -634,6 +634,8 @@ int lace_gpu_ctx::ensure_push(int which, bool *on) {
 int lace_gpu_ctx::limit_reached() {
   for (auto &p : gplans)
     if (p.valid) grid_clear_faces(stream, p);
+  // folds that were left half done: their tags would be taken again
+  if (fold_buf.p) cudaMemsetAsync(fold_buf.p, 0, fold_buf.bytes, stream);
   return DEV_ERR_INTERNAL_LIMIT;
 }
 

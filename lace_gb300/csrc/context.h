@@ -189,7 +189,7 @@ struct lace_gpu_ctx {
   int ensure_push(int which, bool *on);
   int ready_tri(int t1, int t2);
   int ensure_grid(int which);
-  int limit_reached();  // DEV_ERR_INTERNAL_LIMIT, after making the grid plans usable again
+  int limit_reached();  // DEV_ERR_INTERNAL_LIMIT, after making the grid plans and folds usable again
   // z = T2^{-1} T1^{-1} b for two consecutive triangles (L and U, or U^T and L^T)
   int solve_pair(int t1, int t2, const void *b, int in_f32, void *z, int z_f32, bool honor_done, bool prefilled);
   // host plans the autotune built in parallel, keyed (triangle, R, chunks per block)

@@ -2,12 +2,15 @@
 // (src/fgmres_restart.cpp:63-532) and data_fgmres (src/fgmres.cpp:64-517).
 //
 // Modified Gram-Schmidt is sequential in the basis index: the coefficient of
-// v_k is taken from u after v_0..v_{k-1} were removed, so step j needs j+2
-// grid-wide sums one after another.  Two forms of the step after the solves:
-//   k_mgs_step (default): one cooperative kernel, one block per SM keeping
-//     its rows of u in shared memory; each sum is a block sum, a grid barrier
-//     and a fold every block performs in the same order; the second pass
-//     (LACE :336-360) and the rotations run in the same kernel;
+// v_k is taken from u after v_0..v_{k-1} were removed.  Three forms of the step
+// after the solves:
+//   k_mgs_step_ls (default): one cooperative kernel, its blocks keeping their
+//     rows of u and v_j in shared memory; all coefficients from one sum over the
+//     grid (V^T u and V^T v_j) through the inverse of the basis's unit lower Gram
+//     matrix, the norm from a second; the second pass (LACE :336-360) and the
+//     rotations run in the same kernel;
+//   k_mgs_step (where v_j does not fit beside u): the same with j+2 sums one after
+//     another;
 //   one kernel per sum (BCSR operators, u too large for shared memory), each
 //     fusing the previous subtraction with the next dot product in one pass
 //     over u, the second pass in a conditional graph node that the first
