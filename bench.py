@@ -355,7 +355,7 @@ def run_ours(args):
     sweep_gbs = sweep_b / sweep_s / 1e9
     traffic_sweep = profiled_traffic("parilu_sweep_convdiff128.txt", "dram_bytes_per_launch")
     traffic_spmv = profiled_traffic("spmv_convdiff128.txt", "dram_bytes_per_launch")
-    traffic_pair = profiled_traffic("sptrsv_pair_convdiff128.txt", "dram_bytes_per_pair")
+    traffic_pair = profiled_traffic("sptrsv_grid_push.txt", "dram_bytes_per_pair")
     # ---- the bandwidth-bound alternative to the exact solves: k synchronous
     # Jacobi sweeps per triangle (the GPU-native inexact M^-1), the sweeps'
     # rate and what the inexact solves cost in directions
