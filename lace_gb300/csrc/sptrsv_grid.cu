@@ -198,9 +198,10 @@ __device__ void grid_helper(const GridArgs &A, int sy_, int sz_, bool fary, bool
   for (int spins = 0; kb <= ke; ++spins) {
     CT v[4];
     ld_far(src + 4 * kb, v);
+    // all four, on the line or not (see waits below)
     bool ok = true;
 #pragma unroll
-    for (int u = 0; u < 4; ++u) ok = ok && ((unsigned)(4 * kb + u - s) >= (unsigned)g.nx || !unsolved(v[u]));
+    for (int u = 0; u < 4; ++u) ok = ok && !unsolved(v[u]);
     if (ok) {
       st_near(dst + 4 * kb * (int)sizeof(CT), v);
       clear_far(src + 4 * kb);
@@ -429,13 +430,18 @@ __global__ void __launch_bounds__(32 * (kGW + kGHelpers)) k_sptrsv_grid(GridArgs
         ld_face(needY & on, srcY, B.f[0]);
         if (HASZ) ld_face(needZ & on, srcZ, B.f[1]);
       };
-      // whether some entry of block kb's faces that lies on a line is unsolved
+      // Whether some entry of block kb's faces is unsolved, where the lane's line
+      // has a step in the block.  A block with an entry on the line is written
+      // whole, in FP64 by two stores that nothing orders: with the entries off
+      // the line not waited for, the second store could land after the block was
+      // marked unsolved again, and its value be taken for a solved one by the
+      // next tile that uses this face.
       auto waits = [&](auto edge, int kb, const Blk &B) {
         if constexpr (!decltype(edge)::value) return any_unsolved(B.f);
-        bool w = false;
+        bool on = false;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) w |= (unsolved(B.f[0][u]) || unsolved(B.f[1][u])) && valid(4 * kb + u);
-        return w;
+        for (int u = 0; u < 4; ++u) on |= valid(4 * kb + u);
+        return on && any_unsolved(B.f);
       };
       auto poll = [&](auto edge, int kb, Blk &B) {
         for (int spins = 0;; ++spins) {
