@@ -260,6 +260,7 @@ __global__ void __launch_bounds__(32 * (kGW + kGHelpers)) k_sptrsv_grid(GridArgs
   CT *sface = reinterpret_cast<CT *>(smem_g + (size_t)gw * kRing);
   CT *const stage = sface + (size_t)gw * rows * T4;  // the tiles' lines, kGPad values a block
   const int ngroups = (g.sy / g.cy) * (g.sz / g.cz);
+  const bool one_round = ngroups * csize <= (int)gridDim.x;  // a ticket each
   // What does not depend on earlier kernels, then the wait for them.  After it,
   // the next kernel may start in the SMs this one leaves free (it waits for this
   // one's end itself); what a kernel whose predecessor waited here reads of
@@ -553,12 +554,22 @@ __global__ void __launch_bounds__(32 * (kGW + kGHelpers)) k_sptrsv_grid(GridArgs
       asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
       waited = true;
     }
+    // no CTA leaves while another of its cluster may still write to its faces
+    // (the end of a round that another follows is at the loop's top)
+    if (one_round && csize > 1) {
+      __syncwarp();
+      cl.barrier_arrive();
+    }
     if constexpr (!LOWER) {
       __syncthreads();
       if (A.rows_f32) lines_out(0.f);
       else lines_out(0.0);
     }
-    if (ngroups * csize <= (int)gridDim.x) break;  // a ticket each
+    if (one_round) {
+      __syncwarp();
+      if (csize > 1) cl.barrier_wait();
+      break;
+    }
     if constexpr (!LOWER) __syncthreads();
   }
   // the CTA that leaves last re-arms the tickets
