@@ -270,10 +270,14 @@ __global__ void __launch_bounds__(32 * (kGW + kGHelpers)) k_sptrsv_grid(GridArgs
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   }
   const int done = A.done != nullptr ? *(volatile const int *)A.done : 0;
-  const int dirty = *(volatile const int *)A.dirty;
+  // An earlier solve gave up.  The one cluster of a small box sets the flag itself
+  // only after all of its CTAs have read it here; of several clusters another may
+  // have set it meanwhile, so that their CTAs leave or stay together by what
+  // comes with the ticket.
+  const int dirty = ngroups > 1 ? 0 : *(volatile const int *)A.dirty;
   if (A.early && (done || dirty)) asm volatile("griddepcontrol.wait;" ::: "memory");
   if (done) return;  // the same for every CTA
-  if (dirty) {       // an earlier solve gave up
+  if (dirty) {
     if (threadIdx.x == 0) atomicOr(A.status, kStatusSpinTimeout);
     return;
   }
@@ -285,7 +289,14 @@ __global__ void __launch_bounds__(32 * (kGW + kGHelpers)) k_sptrsv_grid(GridArgs
   while (true) {
     int tk = 0;
     if (ngroups > 1) {
-      if (rank == 0 && threadIdx.x == 0) tk = atomicAdd(&A.tickets[0], 1);
+      if (rank == 0 && threadIdx.x == 0) {
+        const int gone = *(volatile const int *)A.dirty;
+        tk = atomicAdd(&A.tickets[0], 1);
+        if (gone) {
+          atomicOr(A.status, kStatusSpinTimeout);
+          tk = ngroups;
+        }
+      }
       __syncwarp();
       tk = __shfl_sync(0xffffffffu, tk, 0);
     }
@@ -296,7 +307,11 @@ __global__ void __launch_bounds__(32 * (kGW + kGHelpers)) k_sptrsv_grid(GridArgs
       cl.sync();
       tk = *(const volatile int *)&s_tile;
     }
-    if (tk >= ngroups) break;  // the same for the whole cluster
+    if (tk >= ngroups) {  // the same for the whole cluster
+      // the kernel after this one may count on the one before it having ended
+      if (!waited) asm volatile("griddepcontrol.wait;" ::: "memory");
+      break;
+    }
     const int gy = g.sy / g.cy;
     const int sy_ = tk % gy * g.cy + ry_, sz_ = tk / gy * g.cz + rz_;  // this CTA's super-tile
     const int ty = sy_ * g.wy + wy, tz = sz_ * g.wz + wz;
