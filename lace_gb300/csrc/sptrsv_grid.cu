@@ -462,7 +462,9 @@ __global__ void __launch_bounds__(32 * (kGW + kGHelpers)) k_sptrsv_grid(GridArgs
       auto poll = [&](auto edge, int kb, Blk &B) {
         for (int spins = 0;; ++spins) {
           faces(1, B);
-          if (!__any_sync(0xffffffffu, waits(edge, kb, B)) || gave_up(spins, A.status, A.dirty)) break;
+          if (!__any_sync(0xffffffffu, waits(edge, kb, B))) break;
+          // the whole warp or none of it: the lanes' steps shuffle
+          if ((spins & 1023) == 1023 && __any_sync(0xffffffffu, gave_up(spins, A.status, A.dirty))) break;
         }
       };
       CT x = (CT)0;
