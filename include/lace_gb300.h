@@ -607,7 +607,10 @@ int lace_gpu_batch_destroy(lace_gpu_batch *batch);
  * device arrays of nrhs vectors of length N = sum n[s], rhs-major: entry i of
  * system s for right-hand side r is at [r*N + row_off[s] + i].  x holds the
  * initial guesses.  iters_out (host, nsys*nrhs, system-major, may be NULL):
- * search directions used per (system, rhs). */
+ * search directions used per (system, rhs).  A pair whose residual is zero has
+ * converged; one whose residual or search direction is not finite (a zero pivot, a
+ * NaN or an infinity in b) ends there, not converged, x updated by the directions
+ * before it only.  DEV_NOTCONVERGED when some pair did not converge. */
 int lace_gpu_batch_solve(lace_gpu_batch *batch, int sweeps, int search_max,
                          int restart_max, double rtol, const double *b,
                          double *x, int *iters_out);

@@ -299,9 +299,11 @@ __global__ void __launch_bounds__(kCT, 1) k_batch_cluster(CBatch P) {
         const double rn2 = total(0), rnorm = sqrt(rn2);
         if (first) s_rtol = P.rtol * rnorm;
         s_step = 0;
-        s_conv = s_live = 0;
-        if (!(rnorm >= s_rtol)) {
+        s_conv = s_live = 0;  // s_conv: 1 converged, -1 not finite
+        if (rnorm < s_rtol || rnorm == 0.0) {
           s_conv = 1;
+        } else if (!(rnorm >= s_rtol)) {
+          s_conv = -1;
         } else {
           const double w0 = xw[buf][0];
           const double dd = mysgn(w0) * rnorm;
@@ -428,10 +430,13 @@ __global__ void __launch_bounds__(kCT, 1) k_batch_cluster(CBatch P) {
           sg[jp1] = -sn * gj;
           sg[j] = cg_ * gj;
           const double resid = fabs(sg[jp1]);
-          s_step = jp1;
-          if (resid < s_rtol || j == m - 1 || !(resid == resid)) {
+          // a column that is not finite, or that the least squares cannot divide by,
+          // ends the solve; the update takes the columns before it
+          const bool bad = !(resid == resid) || !(fabs(Rj[j]) > 0.0);
+          s_step = bad ? j : jp1;
+          if (bad || resid < s_rtol || j == m - 1) {
             s_live = 0;
-            if (resid < s_rtol) s_conv = 1;
+            s_conv = bad ? -1 : resid < s_rtol ? 1 : 0;
           }
         }
         __syncthreads();
@@ -499,7 +504,7 @@ __global__ void __launch_bounds__(kCT, 1) k_batch_cluster(CBatch P) {
     }
     if (rank == 0 && tid == 0) {
       P.iters[sys * P.nrhs + rhs] = iters;
-      P.conv[sys * P.nrhs + rhs] = conv;
+      P.conv[sys * P.nrhs + rhs] = conv > 0;
     }
   }
   cl.sync();  // no CTA leaves while another may still write to it

@@ -234,8 +234,8 @@ __global__ void __launch_bounds__(kPBThreads, 1) k_batch_persist(PBatch P) {
             s_first[c] = 0;
           }
           s_step[c] = 0;
-          if (!(rnorm >= s_rtol[c])) {
-            s_conv[c] = 1;
+          if (!(rnorm >= s_rtol[c]) || rnorm == 0.0) {
+            s_conv[c] = rnorm < s_rtol[c] || rnorm == 0.0 ? 1 : -1;  // -1: not finite
             s_live[c] = 0;
           } else {
             const double w0 = w[0];
@@ -428,10 +428,13 @@ __global__ void __launch_bounds__(kPBThreads, 1) k_batch_persist(PBatch P) {
               sg[c][jp1] = -sn * gj;
               sg[c][j] = cg * gj;
               const double resid = fabs(sg[c][jp1]);
-              s_step[c] = jp1;
-              if (resid < s_rtol[c] || j == m - 1 || !(resid == resid)) {
+              // a column that is not finite, or that the least squares cannot divide
+              // by, ends the solve; the update takes the columns before it
+              const bool bad = !(resid == resid) || !(fabs(Rj[j]) > 0.0);
+              s_step[c] = bad ? j : jp1;
+              if (bad || resid < s_rtol[c] || j == m - 1) {
                 s_live[c] = 0;
-                if (resid < s_rtol[c]) s_conv[c] = 1;
+                s_conv[c] = bad ? -1 : resid < s_rtol[c] ? 1 : 0;
               }
             }
           }
@@ -486,7 +489,7 @@ __global__ void __launch_bounds__(kPBThreads, 1) k_batch_persist(PBatch P) {
       }
       if (tid < nr) {
         P.iters[sys * P.nrhs + rg + tid] = s_iters[tid];
-        P.conv[sys * P.nrhs + rg + tid] = s_conv[tid];
+        P.conv[sys * P.nrhs + rg + tid] = s_conv[tid] > 0;
       }
       __syncthreads();
     }
