@@ -40,7 +40,7 @@ struct lace_gpu_batch {
   // the cluster form: the block-diagonal pattern, and per triangle (0 L, 1 U)
   // the systems' plans one after the other
   std::vector<int> hrow, hcol;
-  int C = 0, K = 2, plan_ct = 0, clusters = 0, gmax[2] = {0, 0}, rbmax = 0;
+  int C = 0, K = 2, plan_ct = 0, plan_m = 0, clusters = 0, gmax[2] = {0, 0}, rbmax = 0;
   size_t slot_bytes = 0, csmem = 0;
   DBuf wptr[2], goff[2], pslot[2], rc[2], dst[2], map[2], dmap[2], cjsys, cjrhs, vals;
 };
@@ -268,7 +268,7 @@ static double persist_cost(const lace_gpu_batch *B, const std::vector<int> &leve
 // The cluster form's plans for value size ct and m directions (C = 0: the
 // batch does not fit it, or the single-CTA form is the better one).
 static int cluster_plan(lace_gpu_batch *B, int m, size_t ct) {
-  if (B->plan_ct == (int)ct && B->m == m) return 0;
+  if (B->plan_ct == (int)ct && B->plan_m == m) return 0;
   B->C = 0;
   B->plan_ct = 0;
   lace_gpu_ctx *c = B->ctx;
@@ -416,6 +416,7 @@ static int cluster_plan(lace_gpu_batch *B, int m, size_t ct) {
     break;
   }
   B->plan_ct = (int)ct;
+  B->plan_m = m;
   return 0;
 }
 
@@ -431,8 +432,8 @@ extern "C" int lace_gpu_batch_destroy(lace_gpu_batch *B) {
 // the per-CTA workspace for search_max m: one CTA per SM (the kernel's
 // register budget), at most one per system
 static int batch_workspace(lace_gpu_batch *B, int m, bool f32) {
-  if (m == B->m && (int)f32 == B->f32 && B->V.p) return 0;
-  B->V.free();
+  if (m == B->m && (int)f32 == B->f32) return 0;
+  B->m = 0;  // until all of it is there
   const int prc = cluster_plan(B, m, f32 ? 4 : 8);
   if (prc) return prc;
   if (B->C) {
@@ -445,10 +446,7 @@ static int batch_workspace(lace_gpu_batch *B, int m, bool f32) {
     rc |= B->Tt.ensure(fb * G * nmax);
     rc |= B->ctl.ensure(4 * (2 + 2 * (size_t)B->nsys * B->nrhs));
     rc |= B->V.ensure(8 * G * (m + 1) * nmax);
-    if (rc) {
-      B->V.free();
-      return DEV_ERR_DEVICE_ALLOC;
-    }
+    if (rc) return DEV_ERR_DEVICE_ALLOC;
     B->m = m;
     B->f32 = f32;
     return 0;
