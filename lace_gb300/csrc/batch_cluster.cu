@@ -29,6 +29,7 @@
 
 #include "context.h"
 #include "krylov_tile.cuh"
+#include "perdevice.h"
 #include "push.cuh"
 
 namespace lace {
@@ -513,9 +514,11 @@ __global__ void __launch_bounds__(kCT, 1) k_batch_cluster(CBatch P) {
 template <typename FT, int K>
 int launch_t(cudaStream_t s, const CBatch &P, int clusters, int *room) {
   const auto fn = k_batch_cluster<FT, K>;
-  static const bool ok =
-      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCSmemMax) == cudaSuccess;
-  if (!ok) return DEV_ERR_UNKNOWN;
+  static PerDevice limits;
+  if (!limits.done([&] {
+        return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCSmemMax) == cudaSuccess;
+      }))
+    return DEV_ERR_UNKNOWN;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(clusters * P.C));
   cfg.blockDim = dim3(kCT);

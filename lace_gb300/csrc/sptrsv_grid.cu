@@ -37,6 +37,7 @@
 #include <cooperative_groups.h>
 
 #include "context.h"
+#include "perdevice.h"
 
 namespace lace {
 
@@ -699,9 +700,11 @@ int helper_rows(const GridShape &g) { return g.wz * (32 >> g.lyl) + (g.nz > 1 ? 
 template <typename CT, bool HASZ, bool LOWER, bool UNIT>
 int launch_t(cudaStream_t s, const GridArgs &a) {
   const auto fn = k_sptrsv_grid<CT, HASZ, LOWER, UNIT>;
-  static const bool ok = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGridSmemMax) ==
-                         cudaSuccess;
-  if (!ok) return DEV_ERR_UNKNOWN;
+  static PerDevice limits;
+  if (!limits.done([&] {
+        return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGridSmemMax) == cudaSuccess;
+      }))
+    return DEV_ERR_UNKNOWN;
   const size_t sm = smem_bytes(a.g, grid_stage_bytes<CT, HASZ, LOWER, UNIT>(), sizeof(CT));
   // the lines' copies want all the warps the registers allow
   const int warps = kGW + kGHelpers, csize = a.g.cy * a.g.cz;

@@ -27,6 +27,7 @@
 #include <cooperative_groups.h>
 
 #include "context.h"
+#include "perdevice.h"
 #include "push.cuh"
 
 namespace lace {
@@ -199,10 +200,12 @@ __global__ void k_push_values(int lanes, int bs, int K, int unit, const int *__r
 template <typename CT, int BS, int K, bool UNIT>
 int launch_t(cudaStream_t s, const PushPlan &p, const PushArgs &a, int *clusters) {
   const auto fn = k_sptrsv_push<CT, BS, K, UNIT>;
-  static const bool ok =
-      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPushSmemMax) == cudaSuccess &&
-      cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
-  if (!ok) return DEV_ERR_UNKNOWN;
+  static PerDevice limits;
+  if (!limits.done([&] {
+        return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPushSmemMax) == cudaSuccess &&
+               cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+      }))
+    return DEV_ERR_UNKNOWN;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)p.C);
   cfg.blockDim = dim3(32 * kPushW);
