@@ -2595,7 +2595,7 @@ extern "C" int lace_gpu_time_arnoldi_step(lace_gpu_ctx *c, int method, int j, in
   // breakdown) must not reach the next operation
   LCHK(cudaMemsetAsync(&a.ctrl->status, 0, 4, c->stream));
   LCHK(cudaMemsetAsync(&a.ctrl->done, 0, 4, c->stream));
-  if (st & kStatusSpinTimeout) return set_err(DEV_ERR_INTERNAL_LIMIT);
+  if (st & kStatusSpinTimeout) return set_err(c->limit_reached());
   *seconds = ms * 1e-3 / reps;
   return DEV_SUCCESS;
 }
