@@ -498,7 +498,7 @@ int lace_gpu_ctx::ensure_plan(int which) {
 int lace_gpu_ctx::try_grid() {
   grid_on = false;
   for (auto &p : gplans) p.valid = false;
-  if (bs || opt.trsv_chunks_per_block > 0 || opt.trsv_rows_per_lane > 0 || n < 2) return 0;
+  if (bs || pinned_schedule() || n < 2) return 0;
   int d[3] = {0, 0, 0};
   const int off = hL.ptr[n] - 1 - hL.ptr[n - 1];  // L's last row without its diagonal
   if (off < 2 || off > 3) return 0;
@@ -548,7 +548,7 @@ int lace_gpu_ctx::try_push(float *ms) {
     pplans[w].valid = false;
     push_unfit[w] = false;
   }
-  if (opt.trsv_chunks_per_block > 0 || opt.trsv_rows_per_lane > 0 || opt.trsv_warps > 0 || opt.trsv_cluster > 0) return 0;
+  if (pinned_schedule()) return 0;
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);

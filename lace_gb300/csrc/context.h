@@ -181,6 +181,10 @@ struct lace_gpu_ctx {
   lace::GridPlan gplans[4];
   lace::DBuf grid_t;  // the vector between the two triangles, in tile order
   int try_grid();
+  // some part of the block-scheduled solves' schedule is pinned
+  bool pinned_schedule() const {
+    return opt.trsv_chunks_per_block > 0 || opt.trsv_rows_per_lane > 0 || opt.trsv_warps > 0 || opt.trsv_cluster > 0;
+  }
   // the solves with pushed values (sptrsv_push.cu), chosen by time; CTAs a triangle (0: none)
   int push_C = 0;
   lace::PushPlan pplans[4];
