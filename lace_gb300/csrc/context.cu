@@ -1785,6 +1785,8 @@ int lace_gpu_ctx::autotune_trsv() {
   if (!rc) rc = try_grid();
   if (rc) return rc;
   if (grid_on) {
+    // with the plans, as the timed solves leave them: precond_enqueue allocates nothing then
+    if ((rc = ready_tri(0, 1))) return rc;
     trsv_tuned = true;
     drop_graphs();
     return 0;
