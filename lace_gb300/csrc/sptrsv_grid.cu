@@ -286,7 +286,7 @@ __global__ void __launch_bounds__(32 * (kGW + kGHelpers)) k_sptrsv_grid(GridArgs
     if constexpr (sizeof(CT) == 4) reinterpret_cast<unsigned *>(sface)[k] = kMark32;
     else reinterpret_cast<unsigned long long *>(sface)[k] = kMark64;
   }
-  bool waited = !A.early;
+  bool waited = !A.early, gone = false;  // gone: this warp gave up a wait
   while (true) {
     int tk = 0;
     if (ngroups > 1) {
@@ -465,7 +465,10 @@ __global__ void __launch_bounds__(32 * (kGW + kGHelpers)) k_sptrsv_grid(GridArgs
           faces(1, B);
           if (!__any_sync(0xffffffffu, waits(edge, kb, B))) break;
           // the whole warp or none of it: the lanes' steps shuffle
-          if ((spins & 1023) == 1023 && __any_sync(0xffffffffu, gave_up(spins, A.status, A.dirty))) break;
+          if ((spins & 1023) == 1023 && __any_sync(0xffffffffu, gave_up(spins, A.status, A.dirty))) {
+            gone = true;
+            break;
+          }
         }
       };
       CT x = (CT)0;
@@ -572,8 +575,10 @@ __global__ void __launch_bounds__(32 * (kGW + kGHelpers)) k_sptrsv_grid(GridArgs
       asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
       waited = true;
     }
-    // no CTA leaves while another of its cluster may still write to its faces
-    // (the end of a round that another follows is at the loop's top)
+    // A tile whose warp has read all its faces has no more of them to come.  A
+    // warp that gave up stays, and its CTA's shared memory with it, until every
+    // warp of the cluster has published.  (Everyone waiting: 128^3 FP32 119.0 us a
+    // pair, like this 116.3.  A round that another follows ends at the loop's top.)
     if (one_round && csize > 1) {
       __syncwarp();
       cl.barrier_arrive();
@@ -585,7 +590,7 @@ __global__ void __launch_bounds__(32 * (kGW + kGHelpers)) k_sptrsv_grid(GridArgs
     }
     if (one_round) {
       __syncwarp();
-      if (csize > 1) cl.barrier_wait();
+      if (gone && csize > 1) cl.barrier_wait();
       break;
     }
     if constexpr (!LOWER) __syncthreads();
