@@ -138,7 +138,9 @@ class Context:
 
     def trsv_schedule(self) -> tuple:
         """(rows per lane, chunks per block, warps per CTA, CTAs per cluster)
-        of the sync-free solves, once the first solve has tuned it."""
+        of the sync-free solves, once the first solve has tuned it; for grid
+        solves (rows of a line, tiles per CTA twice, CTAs per cluster), for
+        solves with pushed values (1, 0, warps per CTA, CTAs)."""
         out = (C.c_int * 4)()
         _chk(self._lib.lace_gpu_get_trsv_schedule(self.h, out), "get_trsv_schedule")
         return tuple(out)

@@ -250,7 +250,7 @@ static double cluster_cost(const lace_gpu_batch *B, const std::vector<int> &leve
 // side and 0.72 us a level, its right-hand sides in lockstep, one job an SM.  It
 // stays the better one where the jobs fill the chip (a level's barrier serves four
 // right-hand sides): 256 systems of 1,024 to 65,536 rows, four right-hand sides,
-// 3.6 s against 5.2 on clusters; the 24 systems above 252 ms against 37.
+// 3.6 s against 5.2 on clusters; the 24 systems above 264 ms against 37.
 static double persist_cost(const lace_gpu_batch *B, const std::vector<int> &levels) {
   double sum = 0.0, top = 0.0;
   for (int s = 0; s < B->nsys; ++s) {

@@ -2087,11 +2087,9 @@ int lace_gpu_ctx::ensure_krylov(int m, bool monitor) {
   return 0;
 }
 
-// A in sliced ELL (slices of 32 rows; within a slice, entry t of all rows
-// together), built from the host copy of the pattern; values gathered from
-// the resident CSR values whenever they change
-// the sliced ELL of a CSR pattern on the host; src[e]: the entry of A whose
-// value entry e takes (null: e itself); pairs: the values as float pairs, too
+// The sliced ELL (slices of 32 rows; within a slice, entry t of all rows together)
+// of a CSR pattern on the host; src[e]: the entry of A whose value entry e takes
+// (null: e itself); pairs: the values as float pairs, too
 int lace_gpu_ctx::build_sell(Sell &S, const int *row, const int *cols, const int *src, bool pairs) {
   S.valid = false;
   // slice widths, their offsets, then the slices, over parallel ranges
@@ -2134,6 +2132,8 @@ int lace_gpu_ctx::build_sell(Sell &S, const int *row, const int *cols, const int
   return 0;
 }
 
+// A in sliced ELL, from the host copy of its pattern; the values gathered from the
+// resident CSR values whenever they change
 int lace_gpu_ctx::ensure_sell() {
   if (bs || (int)hArow.size() != n + 1) return 0;  // CSR uploads only
   if (!sell.valid)

@@ -13,7 +13,8 @@
 //   x update (end of cycle): small least-squares solve + x += Z y (:721-744)
 // k_hh_step runs passes A, B and C of a step as one cooperative kernel (w in
 // shared memory, two grid sums) where the operator is CSR and w fits;
-// the separate passes serve the rest (BCSR, the adjoint, large n).
+// the separate passes serve the rest (BCSR, large n, A^T without room for its
+// sliced ELL).
 // Every kernel returns at once when Control::done is set, so a whole cycle can
 // be launched (or replayed from a CUDA graph) without host round trips.
 #include <math.h>

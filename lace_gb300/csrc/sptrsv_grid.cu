@@ -232,10 +232,10 @@ __host__ __device__ constexpr int grid_stage_bytes() {
   return (3 + (HASZ ? 1 : 0) - (UNIT ? 1 : 0) + (LOWER ? 0 : 1)) * 128 * (int)sizeof(CT);
 }
 
-// Time a pair of triangles (L, then U), before with the block-scheduled kernels
-// and now: 128^3 FP32 228 -> 122 us (DRAM 0.16 GB, the chain is the bound), 64^3
-// FP32 111 -> 64 us, 64^2 FP32 55 -> 28 us; 93 x 70 x 51 in FP64, whose lines are
-// no multiple of a chunk, 12,240 -> 146 us.
+// Time a pair of triangles (L, then U; calls one after the other), with the
+// block-scheduled kernels and with this one: 128^3 FP32 228 -> 116 us (DRAM 85 MB,
+// the chain is the bound), 64^3 116 -> 57 us, 64^2 50 -> 20 us; 128^3 FP64 679 -> 375
+// us; 93 x 70 x 51 in FP64, whose lines are no multiple of a chunk, 12,220 -> 159 us.
 template <typename CT, bool HASZ, bool LOWER, bool UNIT>
 __global__ void __launch_bounds__(32 * (kGW + kGHelpers)) k_sptrsv_grid(GridArgs A) {
   constexpr int D = kGD<CT>;
@@ -756,9 +756,11 @@ bool grid_shape(int n, int d1, int d2, int d3, size_t ct, GridShape &g) {
   // the least time in hand-overs on the way from the first to the last line (in
   // ns, from time stamps of a 128^3 solve: between warps of a CTA, CTAs of a
   // cluster, clusters), then the fewest tiles.  Up to four warps a CTA in FP32
-  // (one a scheduler: 128^3 122 us a pair, two 133, one 161) and two in FP64
-  // (the FP64 unit takes no more); fewer where their lines do not fit its
-  // shared memory.  Clusters of up to eight (128^3: 122 us, four 131).
+  // (one a scheduler: 128^3 122 us a pair, two 133, one 161, when it was first
+  // chosen) and two in FP64 (the FP64 unit takes no more); fewer where their lines
+  // do not fit its shared memory: a CTA holds whole lines, up to about 1,500 rows
+  // in FP32 and 715 in FP64, and longer ones go to the chunks.  Clusters of up to
+  // eight (128^3: 122 us, four 131).
   const long long kWarpHop = 500, kCtaHop = 550, kFarHop = 1800;
   long long best = -1;
   GridShape pick = g;
